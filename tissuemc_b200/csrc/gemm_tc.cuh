@@ -18,9 +18,12 @@
 //   own (issued copies and MMAs finish without help from any other party). Only if a drain wait
 //   runs out too does the CTA free TMEM regardless (so that a later CTA can allocate it) and
 //   report status 2.
-//   The epilogue reads the accumulator with tcgen05.ld, 32 columns per load (warp w owns TMEM
-//   lanes 32w..32w+31, i.e. output rows m0 + 32w + lane), applies the epilogue functor (given the
-//   split index) to each 8 columns and writes global memory.
+//   The epilogue reads the accumulator with tcgen05.ld, 32 columns per load: warp w owns TMEM lanes
+//   32 (w % 4) .. + 31, i.e. output rows, and half w / 4 of the columns. A lane then holds one row,
+//   so storing straight from its registers would touch 32 rows per instruction (it made a
+//   4096 x 512 x 512 layer 18.3 us instead of 10.1). The warp therefore stages each 32 x 32 piece in its 8 KB
+//   of the finished operand ring (16-byte units, swizzled: no bank conflicts) and moves it between
+//   shared and global memory in whole rows of 64 or 128 bytes (EpiTile in mlp.cu).
 #pragma once
 
 #include <cuda.h>
@@ -30,7 +33,8 @@
 
 namespace tmc {
 
-constexpr int kGemmBM = 128, kGemmBK = 64, kGemmThreads = 128, kGemmStages = 3;
+constexpr int kGemmBM = 128, kGemmBK = 64, kGemmThreads = 256, kGemmStages = 3;
+constexpr int kGemmWarpStage = 8192;            // bytes of the ring one warp's epilogue stages through
 constexpr uint32_t kGemmWaitLimit = 1u << 24;   // mbarrier polls before a wait gives up
 constexpr uint32_t kGemmDrainLimit = 1u << 26;  // polls of a wait for this CTA's own issued work
 
@@ -39,17 +43,20 @@ template <int BN> struct GemmSmem {
     static constexpr int b_bytes = BN * 128;
     static constexpr int stage_bytes = a_bytes + b_bytes;
     // alignment slack, the stages, then 2 x kGemmStages + 1 mbarriers, the TMEM address and the
-    // CTA's abort flag
-    static constexpr int bytes = 1024 + kGemmStages * stage_bytes + 128;
+    // CTA's abort flag (128 bytes), and the bias of the tile's columns
+    static constexpr int bytes = 1024 + kGemmStages * stage_bytes + 128 + BN * 4;
 };
 
-// Epilogue functor interface: operator()(split, row, col0, v[8]) for 8 consecutive columns of one
-// row (col0 is a multiple of 8; columns at or beyond N must be ignored by the functor).
+// Epilogue functor interface. `bias` (device pointer or NULL) is added by the functor from the
+// tile's copy in shared memory (zeros where there is none). prefetch(row0, col0, regs) starts
+// loading what the piece at (row0, col0) needs from global memory; piece(split, row0, col0, v,
+// bias, stage, regs) takes 32 consecutive columns of lane's row (row0 + lane) and writes the
+// piece's outputs, ignoring rows >= M and columns >= N. Both are called by whole warps.
 // wait_limit bounds the waits on the other roles (kGemmWaitLimit in production). withhold = 1 is
 // a test of the give-up path: the producer issues no loads, so the issuer's first wait runs out
 // with no copy and no MMA outstanding.
 template <int BN, class Epi>
-__global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a,
+__global__ void __launch_bounds__(kGemmThreads, 2) gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a,
                                                               const __grid_constant__ CUtensorMap tma_b, int M, int N,
                                                               int K, Epi epi, int *status, uint32_t wait_limit,
                                                               int withhold) {
@@ -62,6 +69,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_cons
     uint64_t *acc_bar = empty + kGemmStages;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_bar + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    float *sbias = reinterpret_cast<float *>(base + kGemmStages * GemmSmem<BN>::stage_bytes + 128);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.y * kGemmBM, n0 = blockIdx.x * BN;
@@ -74,6 +82,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_cons
         mbar_init(acc_bar, 1);
         *abort_flag = 0;
     }
+    for (int i = threadIdx.x; i < BN; i += kGemmThreads) sbias[i] = epi.bias && n0 + i < N ? epi.bias[n0 + i] : 0.0f;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -137,6 +146,10 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_cons
         if (lane == 0) atomicCAS(status, 0, 1);
         *abort_flag = 1;
     }
+    // the warp's part of the tile: 32 rows, half of the columns
+    const int row0 = m0 + (warp & 3) * 32, c_first = (warp >> 2) * (BN / 2);
+    typename Epi::Regs regs;
+    epi.prefetch(row0, n0 + c_first, regs);
     // every MMA this CTA issued has completed before TMEM is read or released
     if (!mbar_wait(acc_bar, 0u, wait_limit)) {
         if (lane == 0) atomicCAS(status, 0, 1);
@@ -147,19 +160,18 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(const __grid_cons
     __syncthreads();                 // orders the abort flag: the epilogue runs in every warp or none
     ok = *abort_flag == 0;
     if (ok) {
-        const int row = m0 + warp * 32 + lane;
-        const uint32_t lane_addr = tmem_d + (static_cast<uint32_t>(warp * 32) << 16);
-        static_assert(BN % 32 == 0, "the epilogue reads 32 accumulator columns at a time");
+        // the ring is free: its last bytes were read by the MMAs that acc_bar waited for
+        unsigned char *stage = base + warp * kGemmWarpStage;
+        static_assert((kGemmThreads / 32) * kGemmWarpStage <= kGemmStages * GemmSmem<BN>::stage_bytes, "staging");
+        static_assert(BN == 128 && kGemmThreads == 256, "eight warps: four row groups x two column halves");
+        const uint32_t lane_addr = tmem_d + (static_cast<uint32_t>((warp & 3) * 32) << 16);
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
+        for (int c = c_first; c < c_first + BN / 2; c += 32) {
             float v[32];
             tmem_ld32(lane_addr + static_cast<uint32_t>(c), v);
-            if (row < M) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (n0 + c + 8 * q < N)
-                        epi(static_cast<int>(blockIdx.z), row, n0 + c + 8 * q,
-                            *reinterpret_cast<const float(*)[8]>(v + 8 * q));
+            if (row0 < M && n0 + c < N) {  // warp-uniform
+                epi.piece(static_cast<int>(blockIdx.z), row0, n0 + c, v, sbias + c, stage, regs);
+                if (c + 32 < c_first + BN / 2) epi.prefetch(row0, n0 + c + 32, regs);
             }
         }
     }
