@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_tc_kernel(const __grid_c
     const int kt0 = static_cast<int>(blockIdx.z) * kt_n;
     bool ok = true;
     if (warp == 0) {
-        // ---- producer: the whole warp walks the ring, lane 0 issues
+        // ---- producer: the whole warp walks the ring, one lane issues
         int issued = 0;
         for (int kt = 0; kt < (withhold ? 0 : kt_n); ++kt) {
             const int s = kt % kGemmStages;
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_tc_kernel(const __grid_c
                 ok = false;
                 break;
             }
-            if (lane == 0) {
+            if (elect_one()) {
                 unsigned char *sa = base + s * GemmSmem<BN>::stage_bytes;
                 mbar_arrive_expect_tx(&full[s], GemmSmem<BN>::stage_bytes);
                 tma_load_2d(sa, &tma_a, (kt0 + kt) * kGemmBK, m0, &full[s]);
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_tc_kernel(const __grid_c
                 if (lane == 0) atomicExch(status, 2);
             }
     } else if (warp == 1) {
-        // ---- issuer: the whole warp waits, lane 0 issues the MMAs and the commits
+        // ---- issuer: the whole warp waits, one lane issues the MMAs and the commits
         for (int kt = 0; kt < kt_n; ++kt) {
             const int s = kt % kGemmStages;
             if (!mbar_wait(&full[s], static_cast<uint32_t>((kt / kGemmStages) & 1), wait_limit)) {
@@ -127,19 +127,15 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_tc_kernel(const __grid_c
                 break;
             }
             tc_fence_after();
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint32_t a0 = smem_u32(base + s * GemmSmem<BN>::stage_bytes);
-                const uint32_t b0 = a0 + GemmSmem<BN>::a_bytes;
-#pragma unroll
-                for (int kk = 0; kk < kGemmBK / 16; ++kk)  // 16 bf16 = 32 bytes further along K
-                    umma_bf16(tmem_d, umma_desc_sw128(a0 + kk * 32), umma_desc_sw128(b0 + kk * 32), idesc,
-                              (kt > 0 || kk > 0) ? 1u : 0u);
+                umma_bf16_k64(tmem_d, umma_desc_sw128(a0), umma_desc_sw128(a0 + GemmSmem<BN>::a_bytes), idesc, kt > 0 ? 1u : 0u);
                 umma_commit(&empty[s]);
             }
             __syncwarp();
         }
         // arrives when every MMA issued above has completed, also after a give-up
-        if (lane == 0) umma_commit(acc_bar);
+        if (elect_one()) umma_commit(acc_bar);
         __syncwarp();
     }
     if (!ok) {
