@@ -77,13 +77,6 @@ constexpr int kNoCacheKey = 0x7FFFFFFF;  // the run cache is empty (tally word i
 #define TMC_SWEEP_RUN_CACHE 0
 #endif
 
-// Steps a lane takes per pass of the sweep's loop (the relaunch ballot and the live test once per
-// pass). Measured on the 4096-configuration sweep: 1 1.303 s, 2 1.305 s (the kernel, held to 64
-// registers, spills), 3 1.286 s.
-#ifndef TMC_SWEEP_STEPS_PER_ITER
-#define TMC_SWEEP_STEPS_PER_ITER 3
-#endif
-
 // 1: an ended packet's totals are published when its lane relaunches (as in the single-run kernel)
 // instead of in the step; measured 0.9 % slower with one step per pass and 0.5 % faster with three
 // (within the noise, and the kernel spills), so 0
@@ -115,6 +108,7 @@ template <int FAST, bool TILE, bool PROF> struct SweepCtx {
     static constexpr bool kPublishAtRelaunch = TMC_SWEEP_PUBLISH_AT_RELAUNCH != 0;
 
     __device__ __forceinline__ void refill(Lane &L) const { ring.refill(L, sched, static_cast<int>(P.threads)); }
+    __device__ __forceinline__ void refill2(Lane &L) const { ring.refill2(L, sched, static_cast<int>(P.threads)); }
     __device__ __forceinline__ uint32_t draw(Lane &L) const { return ring.draw(L); }
     __device__ __forceinline__ void skip(Lane &L) const { ring.skip(L); }
     __device__ __forceinline__ uint32_t peek(const Lane &L) const { return ring.peek(L); }
@@ -290,11 +284,12 @@ __device__ __forceinline__ void sweep_body(const SweepParams &P) {
             it_next += take;
         }
         if (ex_mask == 0xffffffffu) break;  // exhausted lanes hold no photon: the warp is done
+        top_up(L, C, alive);
         if (!alive) continue;
         {
             bool ended = false;
 #pragma unroll
-            for (int k = 0; k < TMC_SWEEP_STEPS_PER_ITER; ++k)
+            for (int k = 0; k < kStepsPerPass; ++k)
                 if (!ended) ended = walk_step<FAST>(L, C);
             if (ended) alive = false;
         }

@@ -7,21 +7,6 @@
 
 namespace tmc {
 
-// 1 (default): route a deposit with selects and one generic-address atomic, no divergent paths; 0:
-// branch to the shared or the global atomic. On skin5 the branching form measured 2.1 % slower with
-// a shared core tile and 30 % slower (811 against 624 ms for 1e8 photons) without one, where the
-// lanes of a warp split between the shared last row and column and global memory at most steps.
-#ifndef TMC_DEPOSIT_GENERIC
-#define TMC_DEPOSIT_GENERIC 1
-#endif
-// Steps a lane takes per pass of the persistent loop (the relaunch ballot and the lane's live test
-// once per pass; a lane whose packet ends early in a pass waits out the rest of it). Measured on
-// skin5: 1 597.9 ms, 2 588.5 ms, 3 581.0 ms, 4 682.7 ms (64 registers, the loop body four steps
-// long).
-#ifndef TMC_STEPS_PER_ITER
-#define TMC_STEPS_PER_ITER 3
-#endif
-
 // Shared-memory layout of one block, in 64-bit words (offsets computed identically on the host).
 struct SmemLayout {
     int ring, batch, core_a, lastz_a, lastr_a, rd, tt, layers, total;  // word offsets / total words
@@ -69,11 +54,17 @@ template <int FAST, bool CORE, bool PROF> struct PlainCtx {
     const LayerC *layers;
     unsigned long long *bt;
     int bstride;
-    unsigned long long *s_core, *s_lastz, *s_lastr, *s_rd, *s_tt;
+    // The block's shared words through a generic address, and where the tiles start in them. (An atomic
+    // whose address is known to be shared compiles into a compare-and-swap loop for 64-bit sums: 2,555
+    // SM cycles for a warp on one word, 284 with four lanes on one, 29 with none; the generic form is
+    // one instruction, 32, 14 and 14 cycles.)
+    unsigned long long *words;
+    int at_core, at_lastz, at_lastr, at_rd, at_tt;
     bool cross;
     static constexpr bool kPublishAtRelaunch = true;  // measured 2.4 % faster than in the step
 
     __device__ __forceinline__ void refill(Lane &L) const { ring.refill(L, P.round_keys); }
+    __device__ __forceinline__ void refill2(Lane &L) const { ring.refill2(L, P.round_keys); }
     __device__ __forceinline__ uint32_t draw(Lane &L) const { return ring.draw(L); }
     __device__ __forceinline__ void skip(Lane &L) const { ring.skip(L); }
     __device__ __forceinline__ uint32_t peek(const Lane &L) const { return ring.peek(L); }
@@ -83,26 +74,27 @@ template <int FAST, bool CORE, bool PROF> struct PlainCtx {
         atomicAdd(&bt[L.batch * bstride + slot], v);
     }
 
-    // Deposit into A(r,z) at bin (ir, iz): the shared core tile, the shared cross, or global.
+    // Deposit into A(r,z) at bin (ir, iz): the shared core tile, the shared cross, or global memory, by
+    // one generic-address atomic on the selected word (no divergent paths). The word is an index from
+    // one of two bases: one 64-bit select and one address for whichever it is.
     __device__ __forceinline__ void deposit(int ir, int iz, unsigned long long v) const {
-#if TMC_DEPOSIT_GENERIC
-        // one generic-address atomic on the selected word (no divergent paths)
-        unsigned long long *p = &P.g_arz[static_cast<size_t>(ir) * P.nz + iz];
-        if (cross && ir == P.nr - 1) p = &s_lastr[iz];
-        if (cross && iz == P.nz - 1) p = &s_lastz[ir];
-        if (CORE && ir < P.tr_a && iz < P.tz_a) p = &s_core[ir * P.tz_a + iz];
-        atomicAdd(p, v);
-        return;
-#endif
-        if (CORE && ir < P.tr_a && iz < P.tz_a) {
-            atomicAdd(&s_core[ir * P.tz_a + iz], v);
-        } else if (cross && iz == P.nz - 1) {
-            atomicAdd(&s_lastz[ir], v);
-        } else if (cross && ir == P.nr - 1) {
-            atomicAdd(&s_lastr[iz], v);
-        } else {
-            atomicAdd(&P.g_arz[static_cast<size_t>(ir) * P.nz + iz], v);
+        int idx = ir * P.nz + iz;
+        bool shared = false;
+        if (cross) {
+            if (ir == P.nr - 1) {
+                idx = at_lastr + iz;
+                shared = true;
+            }
+            if (iz == P.nz - 1) {
+                idx = at_lastz + ir;
+                shared = true;
+            }
         }
+        if (CORE && ir < P.tr_a && iz < P.tz_a) {
+            idx = at_core + ir * P.tz_a + iz;
+            shared = true;
+        }
+        atomicAdd((shared ? words : P.g_arz) + idx, v);
     }
 
     // Every deposit goes straight to its word (shared tile or global): a per-lane cache of the last
@@ -121,13 +113,9 @@ template <int FAST, bool CORE, bool PROF> struct PlainCtx {
         const float rr = radius<FAST>(L.xy);
         const int ir = bin_of<FAST>(rr, P.dr, P.inv_dr, P.nr);
         const int ia = bin_of<FAST>(acosf(fminf(fabsf(L.uz), 1.0f)), P.da, P.inv_da, P.na);
-        if (kind == 1) {
-            if (ir < P.tr_rd) atomicAdd(&s_rd[ir * P.na + ia], v);
-            else atomicAdd(&P.g_rd[ir * P.na + ia], v);
-        } else {
-            if (ir < P.tr_tt) atomicAdd(&s_tt[ir * P.na + ia], v);
-            else atomicAdd(&P.g_tt[ir * P.na + ia], v);
-        }
+        const bool top = kind == 1, shared = ir < (top ? P.tr_rd : P.tr_tt);
+        unsigned long long *const base = shared ? words + (top ? at_rd : at_tt) : (top ? P.g_rd : P.g_tt);
+        atomicAdd(base + ir * P.na + ia, v);
     }
 };
 
@@ -159,11 +147,12 @@ __device__ __forceinline__ void walk_body(const WalkParams &P) {
                      reinterpret_cast<const LayerC *>(smem + S.layers),
                      P.batch_smem ? smem + S.batch : P.g_batch,
                      4 + P.nl,
-                     smem + S.core_a,
-                     smem + S.lastz_a,
-                     smem + S.lastr_a,
-                     smem + S.rd,
-                     smem + S.tt,
+                     smem,
+                     S.core_a,
+                     S.lastz_a,
+                     S.lastr_a,
+                     S.rd,
+                     S.tt,
                      P.profiles && P.cross};
 
     const unsigned lane = threadIdx.x & 31u;
@@ -204,11 +193,12 @@ __device__ __forceinline__ void walk_body(const WalkParams &P) {
             }
         }
         if (ex_mask == 0xffffffffu) break;  // exhausted lanes hold no photon: the warp is done
+        top_up(L, C, alive);
         if (!alive) continue;
         {
             bool ended = false;
 #pragma unroll
-            for (int k = 0; k < TMC_STEPS_PER_ITER; ++k)
+            for (int k = 0; k < kStepsPerPass; ++k)
                 if (!ended) ended = walk_step<FAST>(L, C);
             if (ended) alive = false;
         }
@@ -224,25 +214,25 @@ __device__ __forceinline__ void walk_body(const WalkParams &P) {
         }
     }
     for (int i = threadIdx.x; i < (CORE ? P.tr_a * P.tz_a : 0); i += blockDim.x) {
-        const unsigned long long v = C.s_core[i];
+        const unsigned long long v = smem[S.core_a + i];
         if (v) atomicAdd(&P.g_arz[static_cast<size_t>(i / P.tz_a) * P.nz + (i % P.tz_a)], v);
     }
     if (C.cross) {
         for (int i = threadIdx.x; i < P.nr; i += blockDim.x) {
-            const unsigned long long v = C.s_lastz[i];
+            const unsigned long long v = smem[S.lastz_a + i];
             if (v) atomicAdd(&P.g_arz[static_cast<size_t>(i) * P.nz + (P.nz - 1)], v);
         }
         for (int i = threadIdx.x; i < P.nz; i += blockDim.x) {
-            const unsigned long long v = C.s_lastr[i];
+            const unsigned long long v = smem[S.lastr_a + i];
             if (v) atomicAdd(&P.g_arz[static_cast<size_t>(P.nr - 1) * P.nz + i], v);
         }
     }
     for (int i = threadIdx.x; i < P.tr_rd * P.na; i += blockDim.x) {
-        const unsigned long long v = C.s_rd[i];
+        const unsigned long long v = smem[S.rd + i];
         if (v) atomicAdd(&P.g_rd[i], v);
     }
     for (int i = threadIdx.x; i < P.tr_tt * P.na; i += blockDim.x) {
-        const unsigned long long v = C.s_tt[i];
+        const unsigned long long v = smem[S.tt + i];
         if (v) atomicAdd(&P.g_tt[i], v);
     }
 }

@@ -21,16 +21,17 @@
 
 namespace tmc {
 
-// Random words a lane keeps in its shared-memory ring (a power of two). With 16 (the default) the
-// refill is warp-uniform: when any lane of the warp has fewer than the 4 words a step may draw,
-// every lane with room for a block refills too, so the lanes of a warp refill together (0.75
-// refills per step with all 32 lanes busy, against 1 per step with 24 of them when each lane
-// refills on its own; measured 4.3 % faster on skin5). With 8 a lane refills alone. The words each
-// photon consumes, and their order, are the same either way.
-#ifndef TMC_RING_WORDS
-#define TMC_RING_WORDS 16
-#endif
-constexpr uint32_t kRingWords = TMC_RING_WORDS;
+// Steps a lane takes per pass of a kernel's persistent loop: the relaunch ballot, the lane's live test
+// and the random words' top-up once per pass; a lane whose packet ends early in a pass waits out the
+// rest of it. Measured on skin5 with the top-up in every step: 1 597.9 ms, 2 588.5 ms, 3 581.0 ms,
+// 4 682.7 ms (the loop body four steps long).
+constexpr int kStepsPerPass = 3;
+// Random words a lane keeps in its shared-memory ring, and the most a pass may draw (4 a step). Before
+// a pass every lane is topped up to that many, four at a time (one Philox block): while any lane of the
+// warp is short, every lane with room for a block takes one, so the lanes of a warp refill together.
+// The words each photon consumes, and their order, do not depend on it.
+constexpr uint32_t kRingWords = 16, kPassWords = 4u * kStepsPerPass;
+static_assert(kPassWords + 4u <= kRingWords, "a short lane must have room for a block");
 
 // Where a packet keeps its layer's hot constants (Hot): 0 = in registers, loaded on entering a
 // layer; 1 = read from the layer table (shared memory, three 16-byte loads) at every step, which
@@ -39,8 +40,6 @@ constexpr uint32_t kRingWords = TMC_RING_WORDS;
 #define TMC_HOT_SMEM 0
 #endif
 constexpr bool kHotInSmem = TMC_HOT_SMEM != 0;
-
-static_assert(kRingWords == 8 || kRingWords == 16, "ring of 8 or 16 words");
 
 constexpr float kCosZero = 1.0f - 1e-6f;  // physics.hpp:35 (float widening of MCML COSZERO)
 constexpr float kCos90D = 1e-6f;          // physics.hpp:36
@@ -164,8 +163,7 @@ template <int FAST> __device__ __forceinline__ float hg_cos(const Hot &h, float 
 // the scalar form would round it.
 template <int FAST>
 __device__ __forceinline__ void rotate(float2 &uxy, float &uz, float ct, float u) {
-    float st = ffma(-ct, ct, 1.0f);
-    st = st > 0.0f ? m_sqrt<FAST>(st) : 0.0f;
+    const float st = m_sqrt<FAST>(fmaxf(ffma(-ct, ct, 1.0f), 0.0f));
     float sp, cp;
     if constexpr (Math<FAST>::sincos) {
         // psi - pi lies in (-pi, pi), where the SFU sine and cosine are accurate
@@ -186,7 +184,7 @@ __device__ __forceinline__ void rotate(float2 &uxy, float &uz, float ct, float u
         const float2 ixy = ffma2(fmul2(o, f2(oz)), f2(cp), fmul2(f2(-o.y, o.x), f2(sp)));
         const float2 oct = fmul2(o, f2(ct));
         if constexpr (Math<FAST>::sqrt) {
-            const float it = rsqrtf(q);
+            const float it = m_rsqrt<FAST>(q);
             uxy = ffma2(fmul2(f2(st), ixy), f2(it), oct);
             uz = ffma(fmul(fmul(-st, cp), q), it, fmul(oz, ct));
         } else {
@@ -234,15 +232,24 @@ __device__ __forceinline__ void launch(Lane &L, Ctx &C, uint32_t id, int batch, 
     L.run_abs = 0ull;
 }
 
-// Publish an ended packet's per-photon totals (events, anomalies, the weight absorbed in its last
-// layer) into its batch.
-template <class Ctx> __device__ __forceinline__ void finish_photon(const Lane &L, Ctx &C) {
+// Score and publish an ended packet: its exit (check, totals, R_d(r,a) or T_t(r,a)), its events,
+// anomalies and the weight absorbed in its last layer. An ended packet's `steps` says how it ended (0:
+// inside, 1: reflectance, 2: transmittance). Once per pass for every lane that ended in it, instead of
+// in the step with a lane or two: slab (22 steps a photon), 1e7 photons 3.14 -> 2.92 ms.
+template <class Ctx> __device__ __forceinline__ void finish_photon(Lane &L, Ctx &C) {
+    if (L.steps != 0u) {
+        const float n2 = norm2(L.uxy, L.uz);
+        if (!(L.w == L.w) || !(fabsf(fsub(n2, 1.0f)) <= 1e-5f)) ++L.anomalies;
+        const unsigned long long v = to_fixed(L.w);
+        C.batch_add(L, static_cast<int>(L.steps) - 1, v);
+        C.exit(L, static_cast<int>(L.steps), v);
+    }
     C.batch_add(L, 2, static_cast<unsigned long long>(L.events));
     if (L.anomalies) C.batch_add(L, 3, static_cast<unsigned long long>(L.anomalies));
     if (L.run_abs) C.batch_add(L, 4 + L.layer, L.run_abs);
 }
 
-// The first part of a step: refill the random words, the free path (or what is left of it), the
+// The first part of a step: the free path (or what is left of it), the
 // distance to the layer's boundary, and the hop. Returns true when the hop ends on the boundary.
 // The layer constants of the packet's current layer (registers, or the layer table: kHotInSmem).
 template <class Ctx> __device__ __forceinline__ Hot hot_of(const Lane &L, Ctx &C) {
@@ -256,12 +263,6 @@ template <class Ctx> __device__ __forceinline__ Hot hot_of(const Lane &L, Ctx &C
 }
 
 template <int FAST, class Ctx> __device__ __forceinline__ bool step_move(Lane &L, Ctx &C, const Hot &h) {
-    if constexpr (kRingWords == 8) {
-        if (L.wp - L.rp < 4u) C.refill(L);  // a step draws at most 4 words
-    } else {
-        // warp-uniform: the lanes stepping together refill together when any of them is short
-        if (__any_sync(__activemask(), L.wp - L.rp < 4u) && L.wp - L.rp <= kRingWords - 4u) C.refill(L);
-    }
     ++L.steps;
     float s;
     {
@@ -356,12 +357,7 @@ template <int FAST, class Ctx> __device__ __forceinline__ bool step_tail(Lane &L
     // roulette threshold, the step cap (measured 0.4 % faster on skin5 than three tests)
     if (exit_kind != 0 || L.w < kWeightMin || L.steps >= C.step_cap) {
         if (exit_kind) {
-            // ---- score the exit (check, totals, R_d(r,a) or T_t(r,a))
-            const float n2 = norm2(L.uxy, L.uz);
-            if (!(L.w == L.w) || !(fabsf(fsub(n2, 1.0f)) <= 1e-5f)) ++L.anomalies;
-            const unsigned long long v = to_fixed(L.w);
-            C.batch_add(L, exit_kind - 1, v);
-            C.exit(L, exit_kind, v);
+            // scored when the packet is published (finish_photon)
         } else if (L.w < kWeightMin) {
             // ---- roulette (physics.hpp:250-259)
             if (L.w == 0.0f) {
@@ -377,6 +373,7 @@ template <int FAST, class Ctx> __device__ __forceinline__ bool step_tail(Lane &L
             ++L.anomalies;
             died = true;
         }
+        if (died) L.steps = static_cast<uint32_t>(exit_kind);  // how the packet ended (finish_photon)
     }
     if constexpr (!Ctx::kPublishAtRelaunch) {
         if (died) finish_photon(L, C);
@@ -395,6 +392,21 @@ template <int FAST, class Ctx> __device__ __forceinline__ bool walk_step(Lane &L
     if (step_move<FAST>(L, C, h)) step_boundary<FAST>(L, C, exit_kind, died);
     else step_interaction<FAST>(L, C, h);
     return step_tail<FAST>(L, C, exit_kind, died);
+}
+
+// Whole warp, before a pass: top up the random words of the lanes that hold a live packet, by two
+// blocks at once (independent chains of rounds) when all of them have the room. Against a vote and a
+// block in every step: 1e3 photons of skin5 (latency) 1,796 -> 1,758 us, slab 1e7 2.89 -> 2.84 ms, three
+// layers in exact math, 3e5 photons, 1,220 -> 1,166 us.
+template <class Ctx> __device__ __forceinline__ void top_up(Lane &L, Ctx &C, bool alive) {
+    if (__all_sync(0xffffffffu, !alive || L.wp - L.rp <= kRingWords - 8u)) {
+        if (alive) {
+            C.refill2(L);
+        }
+    }
+    while (__any_sync(0xffffffffu, alive && L.wp - L.rp < kPassWords)) {
+        if (alive && L.wp - L.rp <= kRingWords - 4u) C.refill(L);
+    }
 }
 
 // This lane's slot 0 in its block's ring area: each warp has its own region of kRingWords slots,
@@ -431,6 +443,21 @@ struct Ring {
     __device__ __forceinline__ void refill(Lane &L, uint32_t k0, uint32_t k1) const {
         uint32_t b0, b1, b2, b3;
         philox4x32_10(L.id, 0u, L.blk, k0, k1, b0, b1, b2, b3);
+        store(L, b0, b1, b2, b3);
+    }
+    // two blocks at once: two independent chains of rounds
+    __device__ __forceinline__ void refill2(Lane &L, const uint32_t (&rk)[20]) const {
+        uint32_t a0, a1, a2, a3, b0, b1, b2, b3;
+        philox4x32_10_rk(L.id, 0u, L.blk, rk, a0, a1, a2, a3);
+        philox4x32_10_rk(L.id, 0u, L.blk + 1u, rk, b0, b1, b2, b3);
+        store(L, a0, a1, a2, a3);
+        store(L, b0, b1, b2, b3);
+    }
+    __device__ __forceinline__ void refill2(Lane &L, const uint4 *sched, int sched_stride) const {
+        uint32_t a0, a1, a2, a3, b0, b1, b2, b3;
+        philox4x32_10_sched(L.id, 0u, L.blk, sched, sched_stride, a0, a1, a2, a3);
+        philox4x32_10_sched(L.id, 0u, L.blk + 1u, sched, sched_stride, b0, b1, b2, b3);
+        store(L, a0, a1, a2, a3);
         store(L, b0, b1, b2, b3);
     }
     // with a precomputed key schedule (one key for every lane of the launch)
