@@ -161,7 +161,8 @@ __device__ __forceinline__ void walk_body(const WalkParams &P) {
     const uint32_t chunk = static_cast<uint32_t>(P.chunk);
 
     WarpPool pool;                           // warp-uniform photon-id pool
-    unsigned ex_mask = 0u;                   // warp-uniform: lanes with no photon left to take
+    // warp-uniform: lanes with no photon left to take (from the start, those a small run leaves idle)
+    unsigned ex_mask = P.lanes < 32 ? ~0u << P.lanes : 0u;
     bool alive = false;
     bool held = false;  // L holds a photon whose totals are not yet published
     Lane L;

@@ -35,7 +35,7 @@ struct WarpPool {
     TMC_HD bool must_claim(uint32_t n) const { return end - next < n; }
 
     // The id for the lane of rank `rank` (0 .. n - 1) among the n wanting ones; `base` is the
-    // chunk of `chunk` ids (chunk >= 32) claimed when must_claim(n), ignored otherwise. Ids of the
+    // chunk of `chunk` ids (chunk >= n) claimed when must_claim(n), ignored otherwise. Ids of the
     // old pool go first, then those of the new chunk. Call once per lane with the same n and base:
     // the pool advances identically everywhere.
     TMC_HD uint32_t take(uint32_t n, uint32_t rank, uint32_t base, uint32_t chunk) {
