@@ -61,23 +61,26 @@ struct DeviceCtx {
 DeviceCtx g_ctx[kMaxDevices];
 std::mutex g_mu;
 
-// The walk kernel for a launch: fast or exact math, with or without a shared core tile of A(r,z).
-const void *walk_kernel_for(bool fast, bool core, bool profiles = true) {
-    if (!profiles) return fast ? reinterpret_cast<const void *>(walk_kernel_totals<1>)
-                               : reinterpret_cast<const void *>(walk_kernel_totals<0>);
-    if (fast) return core ? reinterpret_cast<const void *>(walk_kernel<1, true>) : reinterpret_cast<const void *>(walk_kernel<1, false>);
-    return core ? reinterpret_cast<const void *>(walk_kernel<0, true>) : reinterpret_cast<const void *>(walk_kernel<0, false>);
+// The walk kernel for a launch: fast or exact math, with or without a shared core tile of A(r,z), with or
+// without profile tallies, and whether the last packets are walked alone.
+template <int FAST, bool ALONE> const void *walk_kernel_of(bool core, bool profiles) {
+    if (!profiles) return reinterpret_cast<const void *>(walk_kernel_totals<FAST, ALONE>);
+    return core ? reinterpret_cast<const void *>(walk_kernel<FAST, true, ALONE>)
+                : reinterpret_cast<const void *>(walk_kernel<FAST, false, ALONE>);
+}
+const void *walk_kernel_for(bool fast, bool core, bool profiles = true, bool alone = false) {
+    if (alone) return fast ? walk_kernel_of<1, true>(core, profiles) : walk_kernel_of<0, true>(core, profiles);
+    return fast ? walk_kernel_of<1, false>(core, profiles) : walk_kernel_of<0, false>(core, profiles);
 }
 
 // Every instantiation may use the device's whole opt-in shared memory per block.
 cudaError_t allow_walk_smem(const cudaDeviceProp &prop) {
-    for (int f = 0; f < 2; ++f)
-        for (int k = 0; k < 3; ++k) {
-            const cudaError_t e = cudaFuncSetAttribute(walk_kernel_for(f != 0, k == 1, k != 2),
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       static_cast<int>(prop.sharedMemPerBlockOptin));
-            if (e != cudaSuccess) return e;
-        }
+    for (int k = 0; k < 16; ++k) {
+        const cudaError_t e = cudaFuncSetAttribute(walk_kernel_for(k & 1, k & 2, k & 4, k & 8),
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   static_cast<int>(prop.sharedMemPerBlockOptin));
+        if (e != cudaSuccess) return e;
+    }
     return cudaSuccess;
 }
 
@@ -133,15 +136,28 @@ uint64_t resident_blocks(const void *kern, const cudaDeviceProp &prop, int threa
     return static_cast<uint64_t>(prop.multiProcessorCount) * static_cast<uint64_t>(std::max(1, occ));
 }
 
+// Whether a run's last packets are walked alone. The kernel that does takes 80 registers, three blocks
+// per SM instead of four, and is 3 to 5 % slower while the device is full; what it saves is the end of the
+// run, as long as its longest photon. Measured with and without, per photons to each of the 151,552
+// resident lanes: slab 1.3 a lane 182 / 210 us, 6.6 411 / 428, 13 698 / 698, 26 1,271 / 1,229, 66 3,005 /
+// 2,844; skin5 1.3 3.06 / 4.46 ms, 6.6 7.25 / 8.20, 13 12.6 / 13.2, 66 55.7 / 54.2. In exact math the
+// accurate functions are most of a step either way: three layers, 0.07 a lane 380 / 501 us, 0.2 480 / 581,
+// 0.66 816 / 773.
+bool walk_ends_alone(const WalkParams &P, const Plan &pl, bool fast) {
+    const uint64_t lanes = static_cast<uint64_t>(pl.grid) * static_cast<uint64_t>(pl.threads);
+    return fast ? P.photons <= 16 * lanes : P.photons <= lanes / 2;
+}
+
 // How a launch spreads its photons: P.lanes and P.chunk, and the grid (returned). Never more blocks than
 // can be resident at once with this plan's shared memory: the kernel is persistent, a second wave would
 // idle. A run whose photons do not fill those is as long as its longest photon, step after step, so the
 // photons go evenly to every SM, to kSmallWarps warps on each before any SM gets more, and a warp's
 // lanes are then not all used: a warp steps faster when its lanes rarely differ (a boundary next to an
 // interaction, an exit, a relaunch). Measured against full warps in as few blocks as hold them, slab:
-// 1e2 photons 76 -> 59 us, 1e4 117 -> 106 us, 3e4 137 -> 116 us; skin5, 1e4: 2.44 -> 1.89 ms. With 16
-// warps per SM 1e4 photons take 109 us and with 32, 116 us; 70,000 take 141 us in two even blocks per SM
-// and 147 us in 274 full ones.
+// 1e2 photons 76 -> 59 us, 1e4 117 -> 106 us, 3e4 137 -> 116 us; skin5, 1e4: 2.44 -> 1.89 ms; 70,000 photons
+// of the slab in two even blocks per SM 141 us, in 274 full ones 147. With the last packets walked alone
+// (8 / 16 / 24 warps per SM): slab 1e4 74.5 / 73.2 / 72.0 us, 3e4 91.1 / 94.8 / 105.9; skin5 3e4 1.56 / 1.74 /
+// 2.01 ms; three layers in exact math 1e4 392 / 442 / 495 us.
 constexpr uint64_t kSmallWarps = 8;
 int walk_grid(WalkParams &P, const Plan &pl, const void *kern, const cudaDeviceProp &prop, size_t smem) {
     const uint64_t warps = static_cast<uint64_t>(pl.threads) / 32, sms = static_cast<uint64_t>(prop.multiProcessorCount);
@@ -370,7 +386,8 @@ void launch_walk(const tmc_run_spec &spec, const tmc_options &opt, DeviceCtx &c,
     const size_t smem = plan_smem_bytes(P);
     if (smem > c.prop.sharedMemPerBlockOptin)
         throw Fail(TMC_BAD_CONFIG, "the tally plan does not fit in shared memory");
-    const void *kern = walk_kernel_for(opt.fast_math != 0, pl.tr_a > 0 && pl.tz_a > 0, P.profiles != 0);
+    const void *kern = walk_kernel_for(opt.fast_math != 0, pl.tr_a > 0 && pl.tz_a > 0, P.profiles != 0,
+                                       walk_ends_alone(P, pl, opt.fast_math != 0));
     const int grid = walk_grid(P, pl, kern, c.prop, smem);
     if (e0) TMC_CUDA(cudaEventRecord(e0, stream));
     if (counter == d_tally + words) {  // one clear for both
@@ -610,7 +627,8 @@ int tmc_b200_run_static(const tmc_run_spec *spec, const tmc_options *opt, tmc_re
         const size_t smem = plan_smem_bytes(P);
         if (smem > d.prop.sharedMemPerBlockOptin)
             throw Fail(TMC_BAD_CONFIG, "the tally plan does not fit in shared memory");
-        const void *kern = walk_kernel_for(opt->fast_math != 0, pl.tr_a > 0 && pl.tz_a > 0, P.profiles != 0);
+        const void *kern = walk_kernel_for(opt->fast_math != 0, pl.tr_a > 0 && pl.tz_a > 0, P.profiles != 0,
+                                           walk_ends_alone(P, pl, opt->fast_math != 0));
         const int grid = walk_grid(P, pl, kern, d.prop, smem);
         // the array keeps the previous call's contents: the counter and the tallies start at zero
         TMC_CUDA(cudaMemsetAsync(d.scratch, 0, (kStaticHeadWords + words) * 8, 0));

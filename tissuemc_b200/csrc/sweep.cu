@@ -160,7 +160,8 @@ struct SweepGraph {
     tmc_sweep_options opt{};
     int cap_cfg = 0, lmax = 0;
     size_t stride = 0;
-    int threads = 256, grid = 0;
+    int threads = 256, grid = 0, sms = 0;
+    bool block = false;  // the block kernel (a block's tile) or the item kernel
     size_t smem = 0;
     cudaStream_t stream = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -221,19 +222,32 @@ std::unique_ptr<SweepGraph> build_graph(int cap, int lmax, const tmc_sweep_optio
               static_cast<size_t>(g->threads / 32) * o.tile_r * o.tile_z * 8;
     cudaDeviceProp prop;
     SW_CUDA(cudaGetDeviceProperties(&prop, o.device));
-    // the kernel for these options: fast or exact math, with or without the per-warp tile, or the
-    // kernel of totals only (no profile tallies)
+    // the kernel for these options: fast or exact math; with profile tallies the block kernel, unless the
+    // options ask for a tile per warp; else the kernel of totals only
     const bool tile = o.profiles && o.tile_r > 0;
+    g->block = o.profiles && !tile;
     const void *kern = !o.profiles ? (o.fast_math ? reinterpret_cast<const void *>(sweep_kernel_totals<1>)
                                                   : reinterpret_cast<const void *>(sweep_kernel_totals<0>))
-                       : o.fast_math ? (tile ? reinterpret_cast<const void *>(sweep_kernel<1, true>)
-                                             : reinterpret_cast<const void *>(sweep_kernel<1, false>))
-                                     : (tile ? reinterpret_cast<const void *>(sweep_kernel<0, true>)
-                                             : reinterpret_cast<const void *>(sweep_kernel<0, false>));
+                       : tile      ? (o.fast_math ? reinterpret_cast<const void *>(sweep_kernel<1>)
+                                                  : reinterpret_cast<const void *>(sweep_kernel<0>))
+                                   : (o.fast_math ? reinterpret_cast<const void *>(sweep_block_kernel<1>)
+                                                  : reinterpret_cast<const void *>(sweep_block_kernel<0>));
+    int bps = 0, tile_words = 0;
+    if (g->block) {
+        // as many resident blocks as the registers allow; the tile takes what they leave of shared memory
+        const size_t ring = 4 * kRingWords * static_cast<size_t>(g->threads), state = sizeof(BlockSweepState) + 16;
+        SW_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(prop.sharedMemPerBlockOptin)));
+        SW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, g->threads, ring + state));
+        const size_t room = prop.sharedMemPerMultiprocessor / static_cast<size_t>(std::max(1, bps)) - prop.reservedSharedMemPerBlock;
+        const size_t words = room > ring + state ? (std::min(room, prop.sharedMemPerBlockOptin) - ring - state) / 8 : 0;
+        tile_words = static_cast<int>(std::min(words, static_cast<size_t>(o.nr) * o.nz));
+        g->smem = ring + state + 8 * static_cast<size_t>(tile_words);
+    }
     SW_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(g->smem)));
-    int bps = 0;
     SW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, g->threads, g->smem));
-    g->grid = prop.multiProcessorCount * std::max(1, bps);
+    g->sms = prop.multiProcessorCount;
+    g->grid = g->sms * std::max(1, bps);
 
     g->off_cfg = align_up(sizeof(SweepHeader));
     g->off_prefix = g->off_cfg + align_up(sizeof(SweepConfigC) * cap);
@@ -274,6 +288,7 @@ std::unique_ptr<SweepGraph> build_graph(int cap, int lmax, const tmc_sweep_optio
     P.threads = static_cast<uint32_t>(g->threads);
     P.tile_r = o.profiles ? o.tile_r : 0;
     P.tile_z = o.profiles ? o.tile_z : 0;
+    P.tile_words = tile_words;
 
     cudaGraph_t graph = nullptr;
     SW_CUDA(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
@@ -345,6 +360,20 @@ uint32_t fill_blob(SweepGraph &g, const tmc_sweep_config *cfgs, int n) {
         g.order[c] = c;
     }
     std::stable_sort(g.order.begin(), g.order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+    // the block kernel: as many blocks as the photons fill, evenly over the SMs, and the lanes a small
+    // sweep needs of each warp; chunks of a sixteenth of a block's share of the estimated work
+    SweepHeader h{};
+    double work = 0.0;
+    uint64_t all = 0;
+    for (int c = 0; c < n; ++c) {
+        work += cost[c] * static_cast<double>(cfgs[c].photons);
+        all += cfgs[c].photons;
+    }
+    const uint64_t sms = static_cast<uint64_t>(g.sms), threads = static_cast<uint64_t>(g.threads);
+    const uint64_t blocks = std::min<uint64_t>(static_cast<uint64_t>(g.grid), sms * ((all + sms * threads - 1) / (sms * threads)));
+    h.blocks = static_cast<uint32_t>(blocks);
+    h.lanes = static_cast<uint32_t>(std::min<uint64_t>(32, (all + blocks * (threads / 32) - 1) / (blocks * (threads / 32))));
+    const double share = work / (16.0 * static_cast<double>(blocks));
     uint64_t total = 0;
     int lbase = 0;
     for (int slot = 0; slot < n; ++slot) {
@@ -363,14 +392,26 @@ uint32_t fill_blob(SweepGraph &g, const tmc_sweep_config *cfgs, int n) {
         k.launch_w = launch_weight(spec);
         k.nl = spec.num_layers;
         k.layer_base = lbase;
+        double chunk = share / cost[g.order[slot]];
+        if (!(chunk > 32.0)) chunk = 32.0;  // also where the estimate is no number
+        k.chunk = static_cast<uint32_t>(std::min({chunk, 16.0 * item, 1073741824.0}));
+        uint32_t k0 = k.k0, k1 = k.k1;
+        for (uint4 &q : k.sched) {  // two rounds' keys each (Weyl increments)
+            q = make_uint4(k0, k1, k0 + 0x9E3779B9u, k1 + 0xBB67AE85u);
+            k0 += 2u * 0x9E3779B9u;
+            k1 += 2u * 0xBB67AE85u;
+        }
         fill_layers(spec, layers + lbase);
         lbase += spec.num_layers;
         prefix[slot] = static_cast<uint32_t>(total);
-        total += (ph + item - 1) / item;
+        const uint32_t each = g.block ? k.chunk : item;
+        total += (static_cast<uint64_t>(ph) + each - 1) / each;
     }
     if (total >= 0xFFFFFFFFull) throw ConfigFailure("too many work items; raise item_photons");
     prefix[n] = static_cast<uint32_t>(total);
-    const SweepHeader h{static_cast<uint32_t>(n), item, sweep_order(static_cast<uint32_t>(total), kSweepBands)};
+    h.n_cfg = static_cast<uint32_t>(n);
+    h.item_photons = item;
+    h.order = sweep_order(static_cast<uint32_t>(total), kSweepBands);
     std::memcpy(g.h_blob, &h, sizeof h);
     return h.order.total;
 }

@@ -22,9 +22,8 @@
 // Optionally (tile_r x tile_z > 0) each warp privatises the first tile_r x tile_z bins of A(r,z) of
 // one configuration, the one of the item it took last, in shared memory: deposits of its lanes'
 // photons of that configuration into those bins are shared-memory atomics. When the warp takes an
-// item of another configuration, its lanes first hand any pending run-cache value for the tile
-// over, then the warp adds the tile's non-zero words into the configuration's global tallies and
-// clears it (integer sums: the totals are the same whichever way they are summed).
+// item of another configuration, it adds the tile's non-zero words into the configuration's global
+// tallies and clears it (integer sums: the totals are the same whichever way they are summed).
 #pragma once
 
 #include "walk_step.cuh"
@@ -39,13 +38,16 @@ struct SweepConfigC {
     float launch_w;                                      // 1 - specular reflectance (float)
     int nl;                                              // layers
     int layer_base;                                      // index of layer 0 in the layer table
-    int pad[3];
+    uint32_t chunk;                                      // photons per chunk of the block kernel
+    int pad[2];
+    uint4 sched[5];                                      // the key's schedule (key_schedule_store)
 };
-static_assert(sizeof(SweepConfigC) == 48, "SweepConfigC layout");
+static_assert(sizeof(SweepConfigC) == 128, "SweepConfigC layout");
 
 // Per-sweep header in device memory (written by the sweep's host-to-device copy, so that one
 // captured graph serves sweeps of different sizes).
 struct SweepHeader {
+    uint32_t blocks, lanes; // block kernel: blocks at work, and lanes of each warp (fewer in a small sweep)
     uint32_t n_cfg;         // configurations
     uint32_t item_photons;  // photons per item (the last item of a configuration may hold fewer)
     SweepOrder order;       // order.total items (configuration c has ceil(photons_c / item_photons))
@@ -66,16 +68,8 @@ struct SweepParams {
     uint32_t step_cap;
     uint32_t threads;
     int tile_r, tile_z;             // per-warp shared tile of A(r,z) (0: none)
+    int tile_words;                 // block kernel: the block's shared tile, the first words of A(r,z)
 };
-
-constexpr int kNoCacheKey = 0x7FFFFFFF;  // the run cache is empty (tally word indices stay below)
-
-// 0 (default): every deposit goes straight to its word; 1: a per-lane run cache merges consecutive
-// deposits into one A(r,z) bin (measured 5 % slower on the 4096-configuration sweep: its branch
-// costs more than the atomics it saves)
-#ifndef TMC_SWEEP_RUN_CACHE
-#define TMC_SWEEP_RUN_CACHE 0
-#endif
 
 // 1: an ended packet's totals are published when its lane relaunches (as in the single-run kernel)
 // instead of in the step; measured 0.9 % slower with one step per pass and 0.5 % faster with three
@@ -95,10 +89,6 @@ template <int FAST, bool TILE, bool PROF> struct SweepCtx {
     int nl;
     const LayerC *layers;
     int t;  // word offset of the configuration's tallies in P.tally (they hold < 2^31 words)
-    // run cache: word index into P.tally of the last A(r,z) bin (or -1 - its index in the warp's
-    // tile), and its pending value
-    int cache_key;
-    unsigned long long cache_val;
     // the warp's tile (warp-uniform): its words, and the configuration it holds (none: 0xFFFFFFFF)
     unsigned long long *tile;
     uint32_t tile_cfg;
@@ -107,52 +97,30 @@ template <int FAST, bool TILE, bool PROF> struct SweepCtx {
     // where an ended packet is published (TMC_SWEEP_PUBLISH_AT_RELAUNCH): in the step by default
     static constexpr bool kPublishAtRelaunch = TMC_SWEEP_PUBLISH_AT_RELAUNCH != 0;
 
-    __device__ __forceinline__ void refill(Lane &L) const { ring.refill(L, sched, static_cast<int>(P.threads)); }
-    __device__ __forceinline__ void refill2(Lane &L) const { ring.refill2(L, sched, static_cast<int>(P.threads)); }
-    __device__ __forceinline__ uint32_t draw(Lane &L) const { return ring.draw(L); }
+    __device__ __forceinline__ void refill(Lane &L) const { ring.refill(L, [&](int q) { return sched[q * static_cast<int>(P.threads)]; }); }
+    __device__ __forceinline__ void refill2(Lane &L) const { ring.refill2(L, [&](int q) { return sched[q * static_cast<int>(P.threads)]; }); }
+    __device__ __forceinline__ float path(const Lane &L, const Hot &h) const { return step_length<FAST>(h, unit_open(ring.peek(L))); }
+    __device__ __forceinline__ float unit(Lane &L) const { return unit_open(ring.draw(L)); }
     __device__ __forceinline__ void skip(Lane &L) const { ring.skip(L); }
-    __device__ __forceinline__ uint32_t peek(const Lane &L) const { return ring.peek(L); }
+    __device__ __forceinline__ void pass(Lane &L, uint32_t n) const { L.rp += n; }
+    __device__ __forceinline__ void scatter(Lane &L, const Hot &h, float dwa) const { scatter_now<FAST>(L, *this, h, dwa); }
+    __device__ __forceinline__ void leave_layer(Lane &) const {}
+    __device__ __forceinline__ void enter_layer(Lane &) const {}
     __device__ __forceinline__ const LayerC &layer(const Lane &, int l) const { return layers[l]; }
     __device__ __forceinline__ int num_layers(const Lane &) const { return nl; }
     __device__ __forceinline__ void batch_add(const Lane &L, int slot, unsigned long long v) const {
         atomicAdd(&P.tally[t + L.batch * bstride + slot], v);
     }
-    __device__ __forceinline__ void deposit(int key, unsigned long long v) const {
-        // negative keys name the warp's tile, which only the TILE instantiation has
-        if (TILE && key < 0) atomicAdd(&tile[-1 - key], v);
-        else atomicAdd(&P.tally[key], v);
-    }
-    __device__ __forceinline__ void absorb(const Lane &L, unsigned long long v) {
+    __device__ __forceinline__ void absorb(float2 xy, float z, unsigned long long v) const {
         if constexpr (!PROF) return;
-        const float rr = radius<FAST>(L.xy);
+        const float rr = radius<FAST>(xy);
         int ir, iz;
-        bins_rz<FAST>(rr, L.z, P.dr, P.dz, P.inv_dr, P.inv_dz, P.nr, P.nz, ir, iz);
-        int key = t + a_off + ir * P.nz + iz;
-        if constexpr (TILE) {
-            if (cfg == tile_cfg && ir < P.tile_r && iz < P.tile_z) key = -1 - (ir * P.tile_z + iz);
-        }
-#if !TMC_SWEEP_RUN_CACHE
-        deposit(key, v);
-        return;
-#endif
-        if (key == cache_key) {
-            cache_val += v;
-        } else {
-            if (cache_key != kNoCacheKey) deposit(cache_key, cache_val);
-            cache_key = key;
-            cache_val = v;
-        }
-    }
-    __device__ __forceinline__ void flush_cache() {
-        if (cache_key != kNoCacheKey) deposit(cache_key, cache_val);
-        cache_key = kNoCacheKey;
+        bins_rz<FAST>(rr, z, P.dr, P.dz, P.inv_dr, P.inv_dz, P.nr, P.nz, ir, iz);
+        if (TILE && cfg == tile_cfg && ir < P.tile_r && iz < P.tile_z) atomicAdd(&tile[ir * P.tile_z + iz], v);
+        else atomicAdd(&P.tally[t + a_off + ir * P.nz + iz], v);
     }
     // Whole warp: hand the tile's sums to the global tallies of its configuration and clear it.
     __device__ __forceinline__ void flush_tile(unsigned lane) {
-        if (cache_key < 0) {  // a pending run-cache value aimed at the tile
-            atomicAdd(&tile[-1 - cache_key], cache_val);
-            cache_key = kNoCacheKey;
-        }
         __syncwarp();
         if (tile_cfg != 0xFFFFFFFFu) {
             for (int i = static_cast<int>(lane); i < P.tile_r * P.tile_z; i += 32) {
@@ -174,12 +142,13 @@ template <int FAST, bool TILE, bool PROF> struct SweepCtx {
     }
 };
 
-// Minimum resident 256-thread blocks per SM the compiler must allow for (0: no bound). A bound of
-// 4 caps the kernel at 64 registers (four blocks per SM instead of three). The step's arithmetic has
-// its rounding pinned (walk.cuh), so the register budget cannot change any photon's path: the
-// tallies stay bit-identical to the single-run kernel's.
+// Minimum resident 256-thread blocks per SM the compiler must allow for (0: no bound). Three allow 80
+// registers; four (64) spilled in the step loop: the block kernel on 4096 configurations 1.44 s with four,
+// 1.22 s with three, 1.24 s without a bound (92 registers, two blocks). The step's arithmetic has its
+// rounding pinned (walk.cuh), so the register budget cannot change any photon's path: the tallies stay
+// bit-identical to the single-run kernel's.
 #ifndef TMC_SWEEP_MIN_BLOCKS
-#define TMC_SWEEP_MIN_BLOCKS 4
+#define TMC_SWEEP_MIN_BLOCKS 3
 #endif
 #if TMC_SWEEP_MIN_BLOCKS > 0
 #define TMC_SWEEP_BOUNDS __launch_bounds__(256, TMC_SWEEP_MIN_BLOCKS)
@@ -188,7 +157,7 @@ template <int FAST, bool TILE, bool PROF> struct SweepCtx {
 #endif
 
 // TILE: the per-warp shared tile of A(r,z) is on (P.tile_r, P.tile_z > 0); the kernel without it
-// is a separate instantiation, so that the tile's bookkeeping costs nothing when it is off.
+// (sweeps of totals only) is a separate instantiation.
 template <int FAST, bool TILE, bool PROF>
 __device__ __forceinline__ void sweep_body(const SweepParams &P) {
     extern __shared__ __align__(16) unsigned long long smem[];
@@ -206,8 +175,6 @@ __device__ __forceinline__ void sweep_body(const SweepParams &P) {
                      1,
                      P.layers,
                      0,
-                     kNoCacheKey,
-                     0ull,
                      // after the key schedules: one tile per warp
                      reinterpret_cast<unsigned long long *>(reinterpret_cast<uint32_t *>(smem) +
                                                             (kRingWords + 20) * P.threads) +
@@ -294,20 +261,257 @@ __device__ __forceinline__ void sweep_body(const SweepParams &P) {
             if (ended) alive = false;
         }
     }
-    C.flush_cache();
     if constexpr (TILE) C.flush_tile(lane);
 }
 
-// The sweep with profile tallies (TILE: with the per-warp shared tile of A(r,z)).
-template <int FAST, bool TILE>
+// The sweep with profile tallies and the per-warp shared tile of A(r,z) that the options ask for.
+template <int FAST>
 __global__ void TMC_SWEEP_BOUNDS sweep_kernel(const __grid_constant__ SweepParams P) {
-    sweep_body<FAST, TILE, true>(P);
+    sweep_body<FAST, true, true>(P);
 }
 
 // The sweep of totals only (no profile tallies).
 template <int FAST>
 __global__ void TMC_SWEEP_BOUNDS sweep_kernel_totals(const __grid_constant__ SweepParams P) {
     sweep_body<FAST, false, false>(P);
+}
+
+// ------------------------------------------------------------------------------ the block kernel
+// The sweep whose blocks work on one configuration at a time, with the leading rows of its A(r,z) (all
+// of a 64 x 64 grid) in shared memory, and walk their last packets alone (walk_step.cuh): a sweep lasts as
+// long as its longest photon, and in a thick, weakly absorbing slab one takes a hundred thousand steps.
+// Against items of 256 photons per warp, every deposit in L2: 97 configurations of 1e3 photons 13.6 ->
+// 3.3 ms, of 1e5 48 -> 42 ms, 1024 of 1e5 166 -> 146 ms, 4096 of 1e4 to 1e6 1.30 -> 1.22 s.
+//
+// A block takes chunks (configuration, first photon, count) from the launch's counter, in the order of
+// the item queue; its warps hand the chunk's photons to their idle lanes. When the chunk runs out the
+// block switches: at the top of a pass all warps meet, the tile's sums go to the old configuration's
+// tallies (unless the next chunk is the same configuration's) and the warps go on. Lanes still walking
+// photons of an earlier configuration are not waited for; their deposits go to global memory. Chunks
+// hold about equal work by the estimate the queue is ordered by (fewer photons where they take more
+// steps), a sixteenth of a block's share, so that a switch (two or three microseconds) stays below a
+// per cent and the launch's end stays even. Warp 0 fetches the next chunk while the block works.
+template <int FAST> struct BlockSweepCtx {
+    const SweepParams &P;
+    Ring ring;
+    uint32_t step_cap;
+    int a_off, rd_off, tt_off, bstride;
+    uint32_t cfg;         // the configuration of this lane's photon
+    const LayerC *layers; // its layers
+    unsigned long long *words;  // the block's tile through a generic address (one native 64-bit atomic)
+    uint32_t tile_cfg;    // the configuration the tile belongs to
+    static constexpr bool kPublishAtRelaunch = true;
+
+    __device__ __forceinline__ uint4 key(int q) const { return __ldg(&P.cfgs[cfg].sched[q]); }
+    __device__ __forceinline__ void refill(Lane &L) const { ring.refill(L, [&](int q) { return key(q); }); }
+    __device__ __forceinline__ void refill2(Lane &L) const { ring.refill2(L, [&](int q) { return key(q); }); }
+    __device__ __forceinline__ void block(uint32_t id, uint32_t blk, uint32_t &w0, uint32_t &w1, uint32_t &w2, uint32_t &w3) const {
+        philox4x32_10_sched(id, 0u, blk, [&](int q) { return key(q); }, w0, w1, w2, w3);
+    }
+    __device__ __forceinline__ uint32_t tag() const { return cfg; }
+    __device__ __forceinline__ void adopt(uint32_t its_cfg) {
+        cfg = its_cfg;
+        layers = P.layers + P.cfgs[cfg].layer_base;
+    }
+    __device__ __forceinline__ float path(const Lane &L, const Hot &h) const { return step_length<FAST>(h, unit_open(ring.peek(L))); }
+    __device__ __forceinline__ float unit(Lane &L) const { return unit_open(ring.draw(L)); }
+    __device__ __forceinline__ void skip(Lane &L) const { ring.skip(L); }
+    __device__ __forceinline__ void pass(Lane &L, uint32_t n) const { L.rp += n; }
+    __device__ __forceinline__ void scatter(Lane &L, const Hot &h, float dwa) const { scatter_now<FAST>(L, *this, h, dwa); }
+    __device__ __forceinline__ void leave_layer(Lane &) const {}
+    __device__ __forceinline__ void enter_layer(Lane &) const {}
+    __device__ __forceinline__ const LayerC &layer(const Lane &, int l) const { return layers[l]; }
+    __device__ __forceinline__ int num_layers(const Lane &) const { return __ldg(&P.cfgs[cfg].nl); }
+    // the sweep's tallies hold fewer than 2^31 words
+    __device__ __forceinline__ int base() const { return static_cast<int>(cfg) * P.stride; }
+    __device__ __forceinline__ void batch_add(const Lane &L, int slot, unsigned long long v) const {
+        atomicAdd(&P.tally[base() + L.batch * bstride + slot], v);
+    }
+    __device__ __forceinline__ void absorb(float2 xy, float z, unsigned long long v) const {
+        const float rr = radius<FAST>(xy);
+        int ir, iz;
+        bins_rz<FAST>(rr, z, P.dr, P.dz, P.inv_dr, P.inv_dz, P.nr, P.nz, ir, iz);
+        const int w = ir * P.nz + iz;
+        const bool shared = cfg == tile_cfg && w < P.tile_words;
+        atomicAdd((shared ? words : P.tally) + (shared ? w : base() + a_off + w), v);
+    }
+    __device__ __forceinline__ void exit(const Lane &L, int kind, unsigned long long v) const {
+        const float rr = radius<FAST>(L.xy);
+        const int ir = bin_of<FAST>(rr, P.dr, P.inv_dr, P.nr);
+        const int ia = P.na > 1 ? bin_of<FAST>(acosf(fminf(fabsf(L.uz), 1.0f)), P.da, P.inv_da, P.na) : 0;
+        atomicAdd(&P.tally[base() + (kind == 1 ? rd_off : tt_off) + ir * P.na + ia], v);
+    }
+};
+
+constexpr uint32_t kNoConfig = 0xFFFFFFFFu;
+
+// The block's state after its rings and tile, in shared memory.
+struct BlockSweepState {
+    uint32_t cfg, next, end;           // the chunk being handed out
+    uint32_t want_switch;              // a warp found it used up
+    uint32_t up_cfg, up_next, up_end;  // the chunk after it (up_cfg = kNoConfig: there is none)
+    uint32_t pad;
+    AloneState alone;
+};
+
+// The block's shared memory after its rings: the tile, then the state.
+__device__ __forceinline__ unsigned long long *block_tile(const SweepParams &P, unsigned long long *smem) {
+    return smem + kRingWords / 2 * P.threads;
+}
+__device__ __forceinline__ BlockSweepState &block_state(const SweepParams &P, unsigned long long *smem) {
+    return *reinterpret_cast<BlockSweepState *>(block_tile(P, smem) + ((P.tile_words + 1) & ~1));
+}
+template <int FAST> __device__ __forceinline__ BlockSweepCtx<FAST> block_ctx(const SweepParams &P, unsigned long long *smem, uint32_t tile_cfg) {
+    const int a_off = P.nb * (4 + P.lmax);
+    return BlockSweepCtx<FAST>{P,
+                               Ring{reinterpret_cast<uint32_t *>(smem) + ring_lane_offset()},
+                               P.step_cap,
+                               a_off,
+                               a_off + P.nr * P.nz,
+                               a_off + P.nr * P.nz + P.nr * P.na,
+                               4 + P.lmax,
+                               0u,
+                               P.layers,
+                               block_tile(P, smem),
+                               tile_cfg};
+}
+
+// Walk the block's parked packets, a warp each (not inlined: the step loop keeps its registers and code).
+template <int FAST> __device__ __noinline__ void sweep_parked(const SweepParams &P, uint32_t tile_cfg, int total) {
+    extern __shared__ __align__(16) unsigned long long smem[];
+    BlockSweepCtx<FAST> C = block_ctx<FAST>(P, smem, tile_cfg);
+    BlockSweepState &S = block_state(P, smem);
+    const unsigned lane = threadIdx.x & 31u;
+    AloneTables &T = alone_tables(smem, threadIdx.x >> 5);
+    for (;;) {
+        const int r = next_parked(S.alone, lane);
+        if (r >= total) break;
+        const Parked &k = alone_tables(smem, static_cast<unsigned>(r) / kAlonePerWarp).parked[r % kAlonePerWarp];
+        Lane M = unpark(k);
+        C.adopt(k.tag);
+        walk_alone<FAST>(M, C, lane, T);
+    }
+}
+
+template <int FAST> __global__ void TMC_SWEEP_BOUNDS sweep_block_kernel(const __grid_constant__ SweepParams P) {
+    extern __shared__ __align__(16) unsigned long long smem[];
+    const SweepHeader &H = *P.hdr;
+    if (blockIdx.x >= H.blocks) return;
+    unsigned long long *const tile = block_tile(P, smem);
+    volatile BlockSweepState &S = block_state(P, smem);
+    BlockSweepCtx<FAST> C = block_ctx<FAST>(P, smem, kNoConfig);
+    const int a_off = C.a_off;
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned lt_mask = (1u << lane) - 1u;
+
+    // warp 0: the block's next chunk
+    const auto fetch = [&]() {
+        if (lane != 0) return;
+        const uint32_t idx = atomicAdd(P.item_counter, 1u);
+        if (idx >= H.order.total) {
+            S.up_cfg = kNoConfig;
+            return;
+        }
+        const uint32_t j = H.order.item(idx), c = sweep_owner(j, H.n_cfg, P.prefix);
+        const uint32_t chunk = P.cfgs[c].chunk, first = (j - P.prefix[c]) * chunk, left = P.cfgs[c].photons - first;
+        S.up_cfg = c;
+        S.up_next = first;
+        S.up_end = first + (left < chunk ? left : chunk);
+    };
+    // whole block: the tile's sums into its configuration's tallies, and clear it
+    const auto flush = [&]() {
+        if (C.tile_cfg == kNoConfig) return;
+        unsigned long long *const a = P.tally + static_cast<size_t>(C.tile_cfg) * P.stride + a_off;
+        for (int i = static_cast<int>(threadIdx.x); i < P.tile_words; i += static_cast<int>(blockDim.x)) {
+            const unsigned long long w = tile[i];
+            if (w) {
+                atomicAdd(a + i, w);
+                tile[i] = 0ull;
+            }
+        }
+    };
+    for (int i = static_cast<int>(threadIdx.x); i < P.tile_words; i += static_cast<int>(blockDim.x)) tile[i] = 0ull;
+    if (threadIdx.x == 0) {
+        S.next = S.end = 0u;
+        S.want_switch = 1u;
+        S.alone.next = 0u;
+    }
+    if (threadIdx.x < 8) S.alone.live[threadIdx.x] = threadIdx.x < P.threads / 32 ? 32 : 0;
+    if (threadIdx.x < 32) fetch();
+    __syncthreads();
+
+    bool done = false;  // block-uniform: no chunk is left to take
+    unsigned ex_mask = H.lanes < 32u ? ~0u << H.lanes : 0u;  // warp-uniform: lanes with no photon left to take
+    bool alive = false;
+    bool held = false;  // L holds an ended photon whose totals are not yet published
+    Lane L;
+    const int alone_at = alone_per_warp<FAST>() * static_cast<int>(P.threads / 32u);
+
+    for (;;) {
+        if (__any_sync(0xffffffffu, S.want_switch != 0u)) {  // set between two switches: every warp comes here once
+            __syncthreads();  // no warp is depositing or handing out photons
+            const uint32_t c = S.up_cfg;
+            if (c == kNoConfig) {
+                done = true;
+            } else {
+                if (c != C.tile_cfg) flush();
+                C.tile_cfg = c;
+            }
+            if (threadIdx.x == 0) {
+                S.cfg = c;
+                S.next = S.up_next;
+                S.end = S.up_end;
+                S.want_switch = 0u;
+            }
+            __syncthreads();
+            if (threadIdx.x < 32 && !done) fetch();
+            __syncwarp();
+        }
+        const unsigned need = ~__ballot_sync(0xffffffffu, alive) & ~ex_mask;
+        if (need) {
+            const bool wants = (need >> lane) & 1u;
+            if (wants && held) {  // the lane's last photon ended: publish it
+                finish_photon(L, C);
+                held = false;
+            }
+            if (done) {
+                ex_mask |= need;
+            } else {
+                const uint32_t n = static_cast<uint32_t>(__popc(need));
+                const uint32_t rank = static_cast<uint32_t>(__popc(need & lt_mask));
+                uint32_t first = 0u;
+                if (lane == 0) first = atomicAdd(const_cast<uint32_t *>(&S.next), n);
+                first = __shfl_sync(0xffffffffu, first, 0);
+                const uint32_t end = S.end, avail = first < end ? end - first : 0u;
+                if (wants && rank < avail) {
+                    C.cfg = C.tile_cfg;
+                    const SweepConfigC &cf = P.cfgs[C.cfg];
+                    C.layers = P.layers + cf.layer_base;
+                    const uint32_t id = first + rank;
+                    launch(L, C, id, batch_of(id, cf.plan_base, cf.plan_extra, cf.plan_bnd), cf.launch_w);
+                    alive = true;
+                    held = true;
+                }
+                if (avail < n && lane == 0) S.want_switch = 1u;
+                __syncwarp();
+            }
+        }
+        if (done) {  // no chunk is left: few enough packets to walk alone?
+            if (lane == 0) S.alone.live[threadIdx.x >> 5] = static_cast<unsigned char>(__popc(~ex_mask));
+            if (live_lanes(S.alone) <= alone_at) break;
+        }
+        top_up(L, C, alive);
+        if (!alive) continue;
+        bool ended = false;
+#pragma unroll
+        for (int k = 0; k < kStepsPerPass; ++k)
+            if (!ended) ended = walk_step<FAST>(L, C);
+        if (ended) alive = false;
+    }
+    // every lane that is not exhausted holds a packet
+    sweep_parked<FAST>(P, C.tile_cfg, park(L, C, ~ex_mask, lane, smem, S.alone));
+    __syncthreads();
+    flush();
 }
 
 // Per-configuration summaries from the integer tallies, in double: R_d(r) per photon (nr values,

@@ -132,15 +132,16 @@ __device__ __forceinline__ void key_schedule_store(uint4 *sched, int stride, uin
     }
 }
 
-// The same rounds with the key schedule read from shared memory (key_schedule_store): for lanes
-// whose keys differ, where a schedule in the parameter bank cannot serve them all.
-__device__ __forceinline__ void philox4x32_10_sched(uint32_t c0, uint32_t c1, uint32_t c2, const uint4 *sched,
-                                                    int stride, uint32_t &o0, uint32_t &o1, uint32_t &o2,
-                                                    uint32_t &o3) {
+// The same rounds with the key schedule in memory: key(q) gives rounds 2q and 2q + 1, as
+// key_schedule_store lays them out (shared memory, or a configuration's table entry). For lanes whose
+// keys differ, where a schedule in the parameter bank cannot serve them all.
+template <class Key>
+__device__ __forceinline__ void philox4x32_10_sched(uint32_t c0, uint32_t c1, uint32_t c2, Key key, uint32_t &o0,
+                                                    uint32_t &o1, uint32_t &o2, uint32_t &o3) {
     uint32_t c3 = 0u;
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
-        const uint4 k = sched[q * stride];
+        const uint4 k = key(q);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint64_t p0 = static_cast<uint64_t>(0xD2511F53u) * c0;

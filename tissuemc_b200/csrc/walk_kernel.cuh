@@ -9,7 +9,7 @@ namespace tmc {
 
 // Shared-memory layout of one block, in 64-bit words (offsets computed identically on the host).
 struct SmemLayout {
-    int ring, batch, core_a, lastz_a, lastr_a, rd, tt, layers, total;  // word offsets / total words
+    int ring, batch, core_a, lastz_a, lastr_a, rd, tt, layers, alone, total;  // word offsets / total words
 };
 
 __host__ __device__ inline SmemLayout smem_layout(const WalkParams &P) {
@@ -37,6 +37,8 @@ __host__ __device__ inline SmemLayout smem_layout(const WalkParams &P) {
     off = (off + 1) & ~1;  // 16-byte alignment for the layer table
     s.layers = off;
     off += (P.nl * static_cast<int>(sizeof(LayerC)) + 7) / 8;
+    s.alone = off;
+    off += static_cast<int>(sizeof(AloneState) / 8);
     s.total = off;
     return s;
 }
@@ -65,9 +67,18 @@ template <int FAST, bool CORE, bool PROF> struct PlainCtx {
 
     __device__ __forceinline__ void refill(Lane &L) const { ring.refill(L, P.round_keys); }
     __device__ __forceinline__ void refill2(Lane &L) const { ring.refill2(L, P.round_keys); }
-    __device__ __forceinline__ uint32_t draw(Lane &L) const { return ring.draw(L); }
+    __device__ __forceinline__ void block(uint32_t id, uint32_t blk, uint32_t &w0, uint32_t &w1, uint32_t &w2, uint32_t &w3) const {
+        philox4x32_10_rk(id, 0u, blk, P.round_keys, w0, w1, w2, w3);
+    }
+    __device__ __forceinline__ uint32_t tag() const { return 0u; }
+    __device__ __forceinline__ void adopt(uint32_t) {}
+    __device__ __forceinline__ float path(const Lane &L, const Hot &h) const { return step_length<FAST>(h, unit_open(ring.peek(L))); }
+    __device__ __forceinline__ float unit(Lane &L) const { return unit_open(ring.draw(L)); }
     __device__ __forceinline__ void skip(Lane &L) const { ring.skip(L); }
-    __device__ __forceinline__ uint32_t peek(const Lane &L) const { return ring.peek(L); }
+    __device__ __forceinline__ void pass(Lane &L, uint32_t n) const { L.rp += n; }
+    __device__ __forceinline__ void scatter(Lane &L, const Hot &h, float dwa) const { scatter_now<FAST>(L, *this, h, dwa); }
+    __device__ __forceinline__ void leave_layer(Lane &) const {}
+    __device__ __forceinline__ void enter_layer(Lane &) const {}
     __device__ __forceinline__ const LayerC &layer(const Lane &, int l) const { return layers[l]; }
     __device__ __forceinline__ int num_layers(const Lane &) const { return P.nl; }
     __device__ __forceinline__ void batch_add(const Lane &L, int slot, unsigned long long v) const {
@@ -100,11 +111,11 @@ template <int FAST, bool CORE, bool PROF> struct PlainCtx {
     // Every deposit goes straight to its word (shared tile or global): a per-lane cache of the last
     // bin (merging consecutive deposits into one bin) measured 4 % slower on skin5, its branch
     // costing more than the atomics it saved.
-    __device__ __forceinline__ void absorb(const Lane &L, unsigned long long v) const {
+    __device__ __forceinline__ void absorb(float2 xy, float z, unsigned long long v) const {
         if constexpr (!PROF) return;
-        const float rr = radius<FAST>(L.xy);
+        const float rr = radius<FAST>(xy);
         int ir, iz;
-        bins_rz<FAST>(rr, L.z, P.dr, P.dz, P.inv_dr, P.inv_dz, P.nr, P.nz, ir, iz);
+        bins_rz<FAST>(rr, z, P.dr, P.dz, P.inv_dr, P.inv_dz, P.nr, P.nz, ir, iz);
         deposit(ir, iz, v);
     }
 
@@ -131,17 +142,8 @@ template <int FAST, bool CORE, bool PROF> struct PlainCtx {
 #endif
 
 template <int FAST, bool CORE, bool PROF>
-__device__ __forceinline__ void walk_body(const WalkParams &P) {
-    extern __shared__ __align__(16) unsigned long long smem[];
-    const SmemLayout S = smem_layout(P);
-    for (int i = S.batch + threadIdx.x; i < S.layers; i += blockDim.x) smem[i] = 0ull;
-    {
-        const float *src = reinterpret_cast<const float *>(P.layers);
-        float *dst = reinterpret_cast<float *>(smem + S.layers);
-        for (int i = threadIdx.x; i < P.nl * static_cast<int>(sizeof(LayerC) / 4); i += blockDim.x) dst[i] = src[i];
-    }
-    __syncthreads();
-    PlainCtx<FAST, CORE, PROF> C{P,
+__device__ __forceinline__ PlainCtx<FAST, CORE, PROF> plain_ctx(const WalkParams &P, const SmemLayout &S, unsigned long long *smem) {
+    return PlainCtx<FAST, CORE, PROF>{P,
                      Ring{reinterpret_cast<uint32_t *>(smem + S.ring) + ring_lane_offset()},
                      P.step_cap,
                      reinterpret_cast<const LayerC *>(smem + S.layers),
@@ -154,6 +156,53 @@ __device__ __forceinline__ void walk_body(const WalkParams &P) {
                      S.rd,
                      S.tt,
                      P.profiles && P.cross};
+}
+
+// Walk the block's parked packets, a warp each; then, in a run so small that its blocks started with that
+// few, what is left of the ids. Not inlined: the step loop's code came out 4 % slower beside it.
+template <int FAST, bool CORE, bool PROF> __device__ __noinline__ void walk_parked(const WalkParams &P, int total) {
+    extern __shared__ __align__(16) unsigned long long smem[];
+    const SmemLayout S = smem_layout(P);
+    PlainCtx<FAST, CORE, PROF> C = plain_ctx<FAST, CORE, PROF>(P, S, smem);
+    AloneState &A = *reinterpret_cast<AloneState *>(smem + S.alone);
+    const unsigned lane = threadIdx.x & 31u;
+    const int warps = static_cast<int>(P.threads) / 32;
+    AloneTables &T = alone_tables(smem + S.ring, threadIdx.x >> 5);
+    for (;;) {
+        Lane M;
+        const int r = next_parked(A, lane);
+        if (r < total) {
+            M = unpark(alone_tables(smem + S.ring, static_cast<unsigned>(r) / kAlonePerWarp).parked[r % kAlonePerWarp]);
+        } else {
+            if (P.lanes > alone_per_warp<FAST>()) break;
+            uint32_t my = 0u;
+            if (lane == 0) my = atomicAdd(P.counter, 1u);
+            my = __shfl_sync(0xffffffffu, my, 0);
+            if (my >= static_cast<uint32_t>(P.photons)) break;
+            const uint32_t id = P.id_base + my;
+            launch(M, C, id, batch_of(id, P.plan_base, P.plan_extra, P.plan_bnd), P.launch_w);
+        }
+        walk_alone<FAST>(M, C, lane, T);
+    }
+}
+
+// ALONE: the run's last packets are walked alone (walk_step.cuh); large runs, whose end is a small part
+// of them, take the kernel without it.
+template <int FAST, bool CORE, bool PROF, bool ALONE>
+__device__ __forceinline__ void walk_body(const WalkParams &P) {
+    extern __shared__ __align__(16) unsigned long long smem[];
+    const SmemLayout S = smem_layout(P);
+    for (int i = S.batch + threadIdx.x; i < S.layers; i += blockDim.x) smem[i] = 0ull;
+    {
+        const float *src = reinterpret_cast<const float *>(P.layers);
+        float *dst = reinterpret_cast<float *>(smem + S.layers);
+        for (int i = threadIdx.x; i < P.nl * static_cast<int>(sizeof(LayerC) / 4); i += blockDim.x) dst[i] = src[i];
+    }
+    volatile AloneState &A = *reinterpret_cast<volatile AloneState *>(smem + S.alone);
+    if (threadIdx.x < 8) A.live[threadIdx.x] = threadIdx.x < P.threads / 32 ? static_cast<unsigned char>(P.lanes) : 0;
+    if (threadIdx.x == 0) A.next = 0u;
+    __syncthreads();
+    PlainCtx<FAST, CORE, PROF> C = plain_ctx<FAST, CORE, PROF>(P, S, smem);
 
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -166,6 +215,7 @@ __device__ __forceinline__ void walk_body(const WalkParams &P) {
     bool alive = false;
     bool held = false;  // L holds a photon whose totals are not yet published
     Lane L;
+    const int alone_at = alone_per_warp<FAST>() * static_cast<int>(P.threads / 32u);
 
     for (;;) {
         // ---- relaunch: lanes without a photon take the next ids from the warp's pool
@@ -193,7 +243,14 @@ __device__ __forceinline__ void walk_body(const WalkParams &P) {
                 held = true;
             }
         }
-        if (ex_mask == 0xffffffffu) break;  // exhausted lanes hold no photon: the warp is done
+        if constexpr (ALONE) {
+            if (ex_mask) {  // ids have run out (or the run is small): few enough packets to walk alone?
+                if (lane == 0) A.live[threadIdx.x >> 5] = static_cast<unsigned char>(__popc(~ex_mask));
+                if (live_lanes(A) <= alone_at) break;
+            }
+        } else {
+            if (ex_mask == 0xffffffffu) break;  // exhausted lanes hold no photon: the warp is done
+        }
         top_up(L, C, alive);
         if (!alive) continue;
         {
@@ -204,6 +261,9 @@ __device__ __forceinline__ void walk_body(const WalkParams &P) {
             if (ended) alive = false;
         }
     }
+
+    // ---- every lane that is not exhausted holds a packet
+    if constexpr (ALONE) walk_parked<FAST, CORE, PROF>(P, park(L, C, ~ex_mask, lane, smem + S.ring, A));
 
     // ---- publish the block's shared tallies into the global ones (integer adds: exact)
     __syncthreads();
@@ -239,15 +299,15 @@ __device__ __forceinline__ void walk_body(const WalkParams &P) {
 }
 
 // The walk of a run with profile tallies (CORE: with a shared core tile of A(r,z)).
-template <int FAST, bool CORE>
+template <int FAST, bool CORE, bool ALONE>
 __global__ void TMC_WALK_BOUNDS walk_kernel(const __grid_constant__ WalkParams P) {
-    walk_body<FAST, CORE, true>(P);
+    walk_body<FAST, CORE, true, ALONE>(P);
 }
 
 // The walk of a run of totals only (no profile tallies).
-template <int FAST>
+template <int FAST, bool ALONE>
 __global__ void TMC_WALK_BOUNDS walk_kernel_totals(const __grid_constant__ WalkParams P) {
-    walk_body<FAST, false, false>(P);
+    walk_body<FAST, false, false, ALONE>(P);
 }
 
 }  // namespace tmc

@@ -70,6 +70,17 @@ struct SweepOrder {
     }
 };
 
+// The configuration c with prefix[c] <= j < prefix[c + 1].
+TMC_HD uint32_t sweep_owner(uint32_t j, uint32_t n_cfg, const uint32_t *prefix) {
+    uint32_t lo = 0u, hi = n_cfg;
+    while (hi - lo > 1u) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (prefix[mid] <= j) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
 // Item `idx` of the sweep's queue (0 <= idx < order.total), taken as order.item(idx).
 // Configuration c owns items prefix[c] .. prefix[c + 1] - 1, each of item_photons photons (its last
 // one fewer when photons_of(c) is not a multiple). Gives the configuration, its first photon and
@@ -79,12 +90,7 @@ TMC_HD void sweep_item(uint32_t idx, const SweepOrder &order, uint32_t item_phot
                        const uint32_t *prefix, PhotonsOf photons_of, uint32_t &cfg, uint32_t &first,
                        uint32_t &end) {
     const uint32_t j = order.item(idx);
-    uint32_t lo = 0u, hi = n_cfg;  // the c with prefix[c] <= j < prefix[c + 1]
-    while (hi - lo > 1u) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (prefix[mid] <= j) lo = mid;
-        else hi = mid;
-    }
+    const uint32_t lo = sweep_owner(j, n_cfg, prefix);
     first = (j - prefix[lo]) * item_photons;
     const uint32_t left = photons_of(lo) - first;
     cfg = lo;
