@@ -419,9 +419,18 @@ TMC_B200_API int tmc_b200_nn_status(int32_t clear);
  *         ystd (log10 R_d(r) per area in the first nbins columns) and weighted by the annulus
  *         areas; rd_mean (optional) gets the members' mean, spread (optional) their sample standard
  *         deviation over the mean, and route[q] = 1 when the spread exceeds threshold (the query
- *         goes to Monte Carlo). */
+ *         goes to Monte Carlo).
+ * encode_f64: encode from float64 features and statistics (the z-score rounded to float32 first).
+ * denormalise: raw outputs in float64 of the members' normalised ones Z[m] (as for gate): Z * std +
+ *         mean per member (out_members: members x n x n_out, optional) and their mean over the members
+ *         in order (out_mean: n x n_out, optional). */
 TMC_B200_API int tmc_b200_nn_encode(const float *feats, const float *mean, const float *stdv, uint16_t *X, int32_t n,
                                     int32_t nf, int32_t ld, void *stream, tmc_status *status);
+TMC_B200_API int tmc_b200_nn_encode_f64(const double *feats, const double *mean, const double *stdv, uint16_t *X,
+                                        int32_t n, int32_t nf, int32_t ld, void *stream, tmc_status *status);
+TMC_B200_API int tmc_b200_nn_denormalise(const float *Z, int32_t members, int64_t member_stride, int32_t ld, int32_t n,
+                                         int32_t n_out, const double *mean, const double *stdv, double *out_members,
+                                         double *out_mean, void *stream, tmc_status *status);
 TMC_B200_API int tmc_b200_nn_gate(const float *Z, int32_t members, int64_t member_stride, int32_t ld,
                                   const float *ymean, const float *ystd, const float *areas, int32_t nbins, int32_t n,
                                   float threshold, float *rd_mean, float *spread, uint8_t *route, void *stream,

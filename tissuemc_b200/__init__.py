@@ -201,6 +201,9 @@ PROTOTYPES = {
     "tmc_b200_nn_to_bf16": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p,
                                            ctypes.c_void_p, ctypes.c_void_p, _P(CStatus)]),
     "tmc_b200_nn_encode": (ctypes.c_int, [ctypes.c_void_p] * 4 + [ctypes.c_int32] * 3 + [ctypes.c_void_p, _P(CStatus)]),
+    "tmc_b200_nn_encode_f64": (ctypes.c_int, [ctypes.c_void_p] * 4 + [ctypes.c_int32] * 3 + [ctypes.c_void_p, _P(CStatus)]),
+    "tmc_b200_nn_denormalise": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64] + [ctypes.c_int32] * 3 +
+                                [ctypes.c_void_p] * 5 + [_P(CStatus)]),
     "tmc_b200_nn_gate": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_int32] +
                          [ctypes.c_void_p] * 3 + [ctypes.c_int32, ctypes.c_int32, ctypes.c_float] +
                          [ctypes.c_void_p] * 4 + [_P(CStatus)]),

@@ -268,10 +268,20 @@ class Ensemble:
         self.step_count = 0  # optimiser steps taken (Adam's bias correction continues across train calls)
 
     def _x(self, X: np.ndarray):
+        """Network inputs of raw features: z-scored in float64, rounded to float32, then to bf16."""
         t = self.torch
-        Xn = np.zeros((len(X), K_IN), dtype=np.float32)
-        Xn[:, :N_FEAT] = (X - self.norm.x_mean) / self.norm.x_std
-        return t.from_numpy(Xn).to(self.dev).to(t.bfloat16)
+        nm = self.norm
+        if len(X) == 0 or X.shape[1:] != (N_FEAT,) or nm.x_mean.shape != (N_FEAT,) or nm.x_std.shape != (N_FEAT,):
+            Xn = np.zeros((len(X), K_IN), dtype=np.float32)
+            Xn[:, :N_FEAT] = (X - nm.x_mean) / nm.x_std  # broadcasts, or says what does not fit
+            return t.from_numpy(Xn).to(self.dev).to(t.bfloat16)
+        # features and statistics in one copy
+        d = t.from_numpy(np.concatenate([np.asarray(X, np.float64).ravel(), nm.x_mean, nm.x_std])).to(self.dev)
+        out = t.empty(len(X), K_IN, dtype=t.bfloat16, device=self.dev)
+        with t.cuda.device(self.dev):
+            _call("tmc_b200_nn_encode_f64", _p(d), _p(d[-2 * N_FEAT:]), _p(d[-N_FEAT:]), _p(out), len(X), N_FEAT, K_IN,
+                  ctypes.c_void_p(t.cuda.current_stream().cuda_stream))
+        return out
 
     def train(self, X: np.ndarray, Y: np.ndarray, epochs: int, lr: float = 1e-3, seed: int = 0,
               lr_final: float = 1e-5, ema: float = 0.0, weight_decay: float = 0.0, graph: bool = True) -> list[float]:
@@ -378,23 +388,34 @@ class Ensemble:
             raise RuntimeError("a tensor-core wait gave up during training")
         return self.history
 
-    def predict_members(self, X: np.ndarray, chunk: int = 65536) -> np.ndarray:
-        """(members, n, 66) raw (de-normalised) outputs."""
-        t = self.torch
-        stream = t.cuda.current_stream().cuda_stream
-        out = np.empty((len(self.members), len(X), N_OUT))
+    def _predict(self, X: np.ndarray, chunk: int, mean: bool) -> np.ndarray:
+        """Raw (de-normalised) outputs in float64: every member's (members, n, 66), or their mean (n, 66)."""
+        t, M = self.torch, len(self.members)
+        out = np.empty((len(X), N_OUT) if mean else (M, len(X), N_OUT))
+        scale = t.from_numpy(np.concatenate([np.broadcast_to(v, N_OUT).astype(np.float64)
+                                             for v in (self.norm.y_mean, self.norm.y_std)])).to(self.dev)
+        f64 = dict(dtype=t.float64, device=self.dev)
         for s in range(0, len(X), chunk):
             Xc = self._x(X[s:s + chunk])
             rows = len(Xc)
-            Z = t.empty(rows, N_OUT_PAD, dtype=t.float32, device=self.dev)
-            for i, m in enumerate(self.members):
-                _ensure_rows(m, rows)
-                m.forward(Xc, rows, stream, Z_out=Z)
-                out[i, s:s + rows] = Z[:, :N_OUT].cpu().numpy() * self.norm.y_std + self.norm.y_mean
+            Z = t.empty(M, rows, N_OUT_PAD, dtype=t.float32, device=self.dev)
+            y = t.empty(*(() if mean else (M,)), rows, N_OUT, **f64)
+            with t.cuda.device(self.dev):
+                stream = t.cuda.current_stream().cuda_stream
+                for i, m in enumerate(self.members):
+                    _ensure_rows(m, rows)
+                    m.forward(Xc, rows, stream, Z_out=Z[i])
+                _call("tmc_b200_nn_denormalise", _p(Z), M, rows * N_OUT_PAD, N_OUT_PAD, rows, N_OUT, _p(scale),
+                      _p(scale[N_OUT:]), _p(None if mean else y), _p(y if mean else None), ctypes.c_void_p(stream))
+            out[..., s:s + rows, :] = y.cpu().numpy()
         return out
 
+    def predict_members(self, X: np.ndarray, chunk: int = 65536) -> np.ndarray:
+        """(members, n, 66) raw (de-normalised) outputs."""
+        return self._predict(X, chunk, False)
+
     def predict(self, X: np.ndarray) -> np.ndarray:
-        return self.predict_members(X).mean(0)
+        return self._predict(X, 65536, True)
 
 
 def _ensure_rows(m: Member, rows: int) -> None:
