@@ -392,6 +392,20 @@ TMC_B200_API int tmc_b200_nn_adam(float *w, const float *g, float *m, float *v, 
                                   float lr_t, const float *lr_dev, float b1, float b2, float eps, float weight_decay,
                                   uint16_t *wb, uint16_t *wt, float *avg, float avg_beta, void *stream,
                                   tmc_status *status);
+/* A training step's passes over all layers of a network in one launch each (at most 8 layers):
+ * weight_grads:   D[q] (M[q] x N[q] float32) = A[q] B[q]^T over K (the batch), split-K with `splits` (1 to 8)
+ *                 partial sums added in order: the bits of matmul_f32_splitk.
+ * colsum_multi:   db[q] = column sums of dZ[q] (M x N[q] bf16, N[q] a multiple of 8): the bits of colsum.
+ * mse_transposes: mse, and the transposes of dZ (ld x M) and of the inputs X (M x k bf16, k x M). */
+TMC_B200_API int tmc_b200_nn_weight_grads(const uint16_t *const *A, const uint16_t *const *B, float *const *D,
+                                          const int32_t *M, const int32_t *N, int32_t count, int32_t K, int32_t splits,
+                                          void *stream, tmc_status *status);
+TMC_B200_API int tmc_b200_nn_colsum_multi(const uint16_t *const *dZ, float *const *db, const int32_t *N, int32_t count,
+                                          int32_t M, void *stream, tmc_status *status);
+TMC_B200_API int tmc_b200_nn_mse_transposes(const float *pred, const float *target, uint16_t *dZ, uint16_t *dZT,
+                                            float *loss, int32_t M, int32_t T, int32_t ld, float scale, const uint16_t *X,
+                                            uint16_t *XT, int32_t k, void *stream, tmc_status *status);
+
 /* One parameter tensor of a many-tensor Adam step (device pointers; rows x cols float32). */
 typedef struct {
     float *w;

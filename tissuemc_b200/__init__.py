@@ -189,6 +189,10 @@ PROTOTYPES = {
     "tmc_b200_nn_colsum_work": (ctypes.c_int32, [ctypes.c_int32]),
     "tmc_b200_nn_mse": (ctypes.c_int, [ctypes.c_void_p] * 4 + [ctypes.c_int32] * 3 + [ctypes.c_float, ctypes.c_void_p,
                                                                                         _P(CStatus)]),
+    "tmc_b200_nn_weight_grads": (ctypes.c_int, [ctypes.c_void_p] * 5 + [ctypes.c_int32] * 3 + [ctypes.c_void_p, _P(CStatus)]),
+    "tmc_b200_nn_colsum_multi": (ctypes.c_int, [ctypes.c_void_p] * 3 + [ctypes.c_int32] * 2 + [ctypes.c_void_p, _P(CStatus)]),
+    "tmc_b200_nn_mse_transposes": (ctypes.c_int, [ctypes.c_void_p] * 5 + [ctypes.c_int32] * 3 + [ctypes.c_float] +
+                                   [ctypes.c_void_p] * 2 + [ctypes.c_int32, ctypes.c_void_p, _P(CStatus)]),
     "tmc_b200_nn_adam": (ctypes.c_int, [ctypes.c_void_p] * 4 + [ctypes.c_int32] * 2 +
                          [ctypes.c_float, ctypes.c_void_p] + [ctypes.c_float] * 4 + [ctypes.c_void_p] * 3 +
                          [ctypes.c_float, ctypes.c_void_p, _P(CStatus)]),

@@ -247,6 +247,17 @@ __device__ __forceinline__ float ld_cluster_f32(const float *p, uint32_t rank) {
         : "memory");
     return v;
 }
+__device__ __forceinline__ float4 ld_cluster_f32x4(const float4 *p, uint32_t rank) {
+    float4 v;
+    asm volatile(
+        "{\n\t.reg .b32 ra;\n\t"
+        "mapa.shared::cluster.u32 ra, %4, %5;\n\t"
+        "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n\t}\n"
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "r"(smem_u32(p)), "r"(rank)
+        : "memory");
+    return v;
+}
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));

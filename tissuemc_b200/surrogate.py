@@ -163,8 +163,6 @@ class Member:
         self.splits = max(1, min(8, batch // 512))
         while (batch // 64) % self.splits:
             self.splits -= 1
-        self.work = torch.empty(self.splits * max(n * k for (k, n) in LAYER_DIMS), **f32)
-        self.colsum_work = torch.empty(lib().tmc_b200_nn_colsum_work(max(n for (_, n) in LAYER_DIMS)), **f32)
         self.L = L
         self._forward_for_training = False  # HT holds the transposed activations of the last forward pass
 
@@ -192,19 +190,20 @@ class Member:
             raise RuntimeError("backward() needs the training forward pass of the same batch first")
         B, s = self.B, ctypes.c_void_p(stream)
         self.loss.zero_()
-        _call("tmc_b200_nn_mse", _p(self.Z[-1]), _p(Y), _p(self.dZ[-1]), _p(self.loss), B, N_OUT, N_OUT_PAD,
-              ctypes.c_float(scale), s)
-        _call("tmc_b200_nn_transpose", _p(X), _p(self.XT), B, K_IN, s)
-        _call("tmc_b200_nn_transpose", _p(self.dZ[-1]), _p(self.dZT[-1]), B, LAYER_DIMS[-1][1], s)
-        for li in range(self.L - 1, -1, -1):
+        _call("tmc_b200_nn_mse_transposes", _p(self.Z[-1]), _p(Y), _p(self.dZ[-1]), _p(self.dZT[-1]), _p(self.loss), B,
+              N_OUT, N_OUT_PAD, ctypes.c_float(scale), _p(X), _p(self.XT), K_IN, s)
+        # every layer's gradient into the layer before, and its transpose for that layer's product
+        for li in range(self.L - 1, 0, -1):
             k, n = LAYER_DIMS[li]
-            prev_T = self.XT if li == 0 else self.HT[li - 1]
-            _call("tmc_b200_nn_matmul_f32_splitk", _p(self.dZT[li]), _p(prev_T), _p(self.gW[li]), _p(self.work),
-                  n, k, B, self.splits, s)
-            _call("tmc_b200_nn_colsum", _p(self.dZ[li]), _p(self.gb[li]), B, n, _p(self.colsum_work), s)
-            if li > 0:  # the gradient into the previous layer, and its transpose for that layer's product
-                _call("tmc_b200_nn_backward_data", _p(self.dZ[li]), _p(self.WT[li]), _p(self.Z[li - 1]),
-                      _p(self.dZ[li - 1]), _p(self.dZT[li - 1]), B, k, n, s)
+            _call("tmc_b200_nn_backward_data", _p(self.dZ[li]), _p(self.WT[li]), _p(self.Z[li - 1]),
+                  _p(self.dZ[li - 1]), _p(self.dZT[li - 1]), B, k, n, s)
+        # then every layer's weight gradient, and every bias gradient, in one launch each
+        arr = lambda ts: (ctypes.c_void_p * self.L)(*[t.data_ptr() for t in ts])  # noqa: E731
+        outs = (ctypes.c_int32 * self.L)(*[n for (_, n) in LAYER_DIMS])
+        ins = (ctypes.c_int32 * self.L)(*[k for (k, _) in LAYER_DIMS])
+        _call("tmc_b200_nn_weight_grads", arr(self.dZT), arr([self.XT, *self.HT]), arr(self.gW), outs, ins, self.L, B,
+              self.splits, s)
+        _call("tmc_b200_nn_colsum_multi", arr(self.dZ), arr(self.gb), outs, self.L, B, s)
 
     def adam(self, stream: int, lr_t: float = 0.0, lr_dev=None, b1=0.9, b2=0.999, eps=1e-8, wd=0.0, avg=None,
              ema: float = 0.0):
