@@ -77,6 +77,7 @@ __device__ __forceinline__ GemmCta<BN> gemm_begin(unsigned char *raw, const floa
         mbar_init(g.acc_bar, 1);
         *g.abort_flag = 0;
     }
+    wait_for_inputs();
     for (int i = threadIdx.x; i < BN; i += kGemmThreads) g.sbias[i] = bias && n0 + i < N ? bias[n0 + i] : 0.0f;
     tc_fence_before();
     __syncthreads();
@@ -238,6 +239,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) wgrad_kernel(const __grid_con
     const int kt_n = K / kGemmBK / splits;
     gemm_products<BN>(g, &P.a[q], &P.b[q], m0, n0, split * kt_n, kt_n, status, kGemmWaitLimit, 0);
     const bool ok = gemm_done<BN>(g, status, kGemmWaitLimit);
+    dependents_may_start();
     // the partial tile in the finished ring: row r at 512 r, its 16-byte unit u at place u ^ (r % 8)
     static_assert(kGemmBM * BN * 4 <= kGemmStages * GemmSmem<BN>::stage_bytes, "the tile fits the ring");
     const auto unit = [&](int r, int u) { return reinterpret_cast<float4 *>(g.base + r * (BN * 4) + ((u ^ (r & 7)) << 4)); };
