@@ -251,12 +251,12 @@ __device__ __forceinline__ void sweep_body(const SweepParams &P) {
             it_next += take;
         }
         if (ex_mask == 0xffffffffu) break;  // exhausted lanes hold no photon: the warp is done
-        top_up(L, C, alive);
+        top_up<FAST>(L, C, alive);
         if (!alive) continue;
         {
             bool ended = false;
 #pragma unroll
-            for (int k = 0; k < kStepsPerPass; ++k)
+            for (int k = 0; k < steps_per_pass<FAST>(); ++k)
                 if (!ended) ended = walk_step<FAST>(L, C);
             if (ended) alive = false;
         }
@@ -500,11 +500,11 @@ template <int FAST> __global__ void TMC_SWEEP_BOUNDS sweep_block_kernel(const __
             if (lane == 0) S.alone.live[threadIdx.x >> 5] = static_cast<unsigned char>(__popc(~ex_mask));
             if (live_lanes(S.alone) <= alone_at) break;
         }
-        top_up(L, C, alive);
+        top_up<FAST>(L, C, alive);
         if (!alive) continue;
         bool ended = false;
 #pragma unroll
-        for (int k = 0; k < kStepsPerPass; ++k)
+        for (int k = 0; k < steps_per_pass<FAST>(); ++k)
             if (!ended) ended = walk_step<FAST>(L, C);
         if (ended) alive = false;
     }

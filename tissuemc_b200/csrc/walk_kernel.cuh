@@ -251,12 +251,12 @@ __device__ __forceinline__ void walk_body(const WalkParams &P) {
         } else {
             if (ex_mask == 0xffffffffu) break;  // exhausted lanes hold no photon: the warp is done
         }
-        top_up(L, C, alive);
+        top_up<FAST>(L, C, alive);
         if (!alive) continue;
         {
             bool ended = false;
 #pragma unroll
-            for (int k = 0; k < kStepsPerPass; ++k)
+            for (int k = 0; k < steps_per_pass<FAST>(); ++k)
                 if (!ended) ended = walk_step<FAST>(L, C);
             if (ended) alive = false;
         }

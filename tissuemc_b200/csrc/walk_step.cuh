@@ -28,15 +28,15 @@ namespace tmc {
 
 // Steps a lane takes per pass of a kernel's persistent loop: the relaunch ballot, the lane's live test
 // and the random words' top-up once per pass; a lane whose packet ends early in a pass waits out the
-// rest of it. Measured on skin5 with the top-up in every step: 1 597.9 ms, 2 588.5 ms, 3 581.0 ms,
-// 4 682.7 ms (the loop body four steps long).
-constexpr int kStepsPerPass = 3;
-// Random words a lane keeps in its shared-memory ring, and the most a pass may draw (4 a step). Before
-// a pass every lane is topped up to that many, four at a time (one Philox block): while any lane of the
+// rest of it. Fast math, skin5, 2e7 photons: 2 107.6 ms, 3 105.4 ms (4: a sixth slower, the loop body four
+// steps long). Exact math, whose step is
+// twice as long, three layers, 3e6 photons: 1 4.86 ms, 2 4.90 ms, 3 5.51 ms; slab, 3e5: 475, 444, 459 us.
+template <int FAST> __device__ __forceinline__ constexpr int steps_per_pass() { return FAST ? 3 : 2; }
+// Random words a lane keeps in its shared-memory ring. Before a pass every lane is topped up to the most
+// that the pass may draw (4 a step), four at a time (one Philox block): while any lane of the
 // warp is short, every lane with room for a block takes one, so the lanes of a warp refill together.
 // The words each photon consumes, and their order, do not depend on it.
-constexpr uint32_t kRingWords = 16, kPassWords = 4u * kStepsPerPass;
-static_assert(kPassWords + 4u <= kRingWords, "a short lane must have room for a block");
+constexpr uint32_t kRingWords = 16;
 
 constexpr float kCosZero = 1.0f - 1e-6f;  // physics.hpp:35 (float widening of MCML COSZERO)
 constexpr float kCos90D = 1e-6f;          // physics.hpp:36
@@ -422,7 +422,9 @@ template <int FAST, class Ctx> __device__ __forceinline__ bool walk_step(Lane &L
 // blocks at once (independent chains of rounds) when all of them have the room. Against a vote and a
 // block in every step: 1e3 photons of skin5 (latency) 1,796 -> 1,758 us, slab 1e7 2.89 -> 2.84 ms, three
 // layers in exact math, 3e5 photons, 1,220 -> 1,166 us.
-template <class Ctx> __device__ __forceinline__ void top_up(Lane &L, Ctx &C, bool alive) {
+template <int FAST, class Ctx> __device__ __forceinline__ void top_up(Lane &L, Ctx &C, bool alive) {
+    constexpr uint32_t kPassWords = 4u * steps_per_pass<FAST>();
+    static_assert(kPassWords + 4u <= kRingWords, "a short lane must have room for a block");
     if (__all_sync(0xffffffffu, !alive || L.wp - L.rp <= kRingWords - 8u)) {
         if (alive) {
             C.refill2(L);
