@@ -361,7 +361,11 @@ uint32_t fill_blob(SweepGraph &g, const tmc_sweep_config *cfgs, int n) {
     }
     std::stable_sort(g.order.begin(), g.order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
     // the block kernel: as many blocks as the photons fill, evenly over the SMs, and the lanes a small
-    // sweep needs of each warp; chunks of a sixteenth of a block's share of the estimated work
+    // sweep needs of each warp; chunks of at most a block's share of the estimated work and of 8 items' photons
+    // (2,048). Smaller chunks scatter a configuration's long photons over blocks that soon work on another
+    // one: 97 configurations of 1e5 photons in chunks of at most 512 / 1,024 / 2,048 / 4,096 photons 36.5 / 28.6 /
+    // 20.8 / 23.1 ms, 300 of 1e4 to 1e6 140 / 112 / 92 / 98 ms, 4096 of those 1.45 / 1.35 / 1.23 / 1.22 s; with a
+    // sixteenth of a block's share 41.5, 129 ms and 1.22 s.
     SweepHeader h{};
     double work = 0.0;
     uint64_t all = 0;
@@ -373,7 +377,7 @@ uint32_t fill_blob(SweepGraph &g, const tmc_sweep_config *cfgs, int n) {
     const uint64_t blocks = std::min<uint64_t>(static_cast<uint64_t>(g.grid), sms * ((all + sms * threads - 1) / (sms * threads)));
     h.blocks = static_cast<uint32_t>(blocks);
     h.lanes = static_cast<uint32_t>(std::min<uint64_t>(32, (all + blocks * (threads / 32) - 1) / (blocks * (threads / 32))));
-    const double share = work / (16.0 * static_cast<double>(blocks));
+    const double share = work / static_cast<double>(blocks);
     uint64_t total = 0;
     int lbase = 0;
     for (int slot = 0; slot < n; ++slot) {
@@ -394,7 +398,7 @@ uint32_t fill_blob(SweepGraph &g, const tmc_sweep_config *cfgs, int n) {
         k.layer_base = lbase;
         double chunk = share / cost[g.order[slot]];
         if (!(chunk > 32.0)) chunk = 32.0;  // also where the estimate is no number
-        k.chunk = static_cast<uint32_t>(std::min({chunk, 16.0 * item, 1073741824.0}));
+        k.chunk = static_cast<uint32_t>(std::min({chunk, 8.0 * item, 1073741824.0}));
         uint32_t k0 = k.k0, k1 = k.k1;
         for (uint4 &q : k.sched) {  // two rounds' keys each (Weyl increments)
             q = make_uint4(k0, k1, k0 + 0x9E3779B9u, k1 + 0xBB67AE85u);

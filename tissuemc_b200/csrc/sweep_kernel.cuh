@@ -281,16 +281,15 @@ __global__ void TMC_SWEEP_BOUNDS sweep_kernel_totals(const __grid_constant__ Swe
 // of a 64 x 64 grid) in shared memory, and walk their last packets alone (walk_step.cuh): a sweep lasts as
 // long as its longest photon, and in a thick, weakly absorbing slab one takes a hundred thousand steps.
 // Against items of 256 photons per warp, every deposit in L2: 97 configurations of 1e3 photons 13.6 ->
-// 3.3 ms, of 1e5 48 -> 42 ms, 1024 of 1e5 166 -> 146 ms, 4096 of 1e4 to 1e6 1.30 -> 1.22 s.
+// 3.3 ms, of 1e5 48 -> 21 ms, 1024 of 1e5 166 -> 135 ms, 4096 of 1e4 to 1e6 1.30 -> 1.23 s.
 //
 // A block takes chunks (configuration, first photon, count) from the launch's counter, in the order of
 // the item queue; its warps hand the chunk's photons to their idle lanes. When the chunk runs out the
 // block switches: at the top of a pass all warps meet, the tile's sums go to the old configuration's
 // tallies (unless the next chunk is the same configuration's) and the warps go on. Lanes still walking
-// photons of an earlier configuration are not waited for; their deposits go to global memory. Chunks
-// hold about equal work by the estimate the queue is ordered by (fewer photons where they take more
-// steps), a sixteenth of a block's share, so that a switch (two or three microseconds) stays below a
-// per cent and the launch's end stays even. Warp 0 fetches the next chunk while the block works.
+// photons of an earlier configuration are not waited for; their deposits go to global memory. A chunk
+// holds at most a block's share of the work, by the estimate the queue is ordered by (sweep.cu); a switch
+// takes two or three microseconds. Warp 0 fetches the next chunk while the block works.
 template <int FAST> struct BlockSweepCtx {
     const SweepParams &P;
     Ring ring;
