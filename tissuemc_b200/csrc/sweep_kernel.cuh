@@ -5,6 +5,9 @@
 // configuration, so a configuration's tallies are bit for bit those of a single run with the
 // same seed, photons, batches and grid.
 //
+// A sweep with profile tallies runs in sweep_block_kernel (below, with its own comment), unless the
+// options ask for a tile of A(r,z) per warp; what follows here is the kernel for that and for totals only.
+//
 // Work is a queue of items (configuration, first photon, count): configuration c's photons in
 // chunks of item_photons, numbered through a prefix sum and taken band by band, in a strided
 // permutation inside each band (work_queue.cuh, SweepOrder), so that the warps at work at any
