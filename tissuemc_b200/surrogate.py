@@ -270,7 +270,7 @@ class Ensemble:
         """Network inputs of raw features: z-scored in float64, rounded to float32, then to bf16."""
         t = self.torch
         nm = self.norm
-        if len(X) == 0 or X.shape[1:] != (N_FEAT,) or nm.x_mean.shape != (N_FEAT,) or nm.x_std.shape != (N_FEAT,):
+        if len(X) == 0 or np.shape(X)[1:] != (N_FEAT,) or not _float64_vectors(N_FEAT, X, nm.x_mean, nm.x_std):
             Xn = np.zeros((len(X), K_IN), dtype=np.float32)
             Xn[:, :N_FEAT] = (X - nm.x_mean) / nm.x_std  # broadcasts, or says what does not fit
             return t.from_numpy(Xn).to(self.dev).to(t.bfloat16)
@@ -389,10 +389,11 @@ class Ensemble:
 
     def _predict(self, X: np.ndarray, chunk: int, mean: bool) -> np.ndarray:
         """Raw (de-normalised) outputs in float64: every member's (members, n, 66), or their mean (n, 66)."""
-        t, M = self.torch, len(self.members)
+        t, M, nm = self.torch, len(self.members), self.norm
+        if not _float64_vectors(N_OUT, np.float32(0), nm.y_std, nm.y_mean):
+            return self._predict_members_numpy(X, chunk).mean(0) if mean else self._predict_members_numpy(X, chunk)
         out = np.empty((len(X), N_OUT) if mean else (M, len(X), N_OUT))
-        scale = t.from_numpy(np.concatenate([np.broadcast_to(v, N_OUT).astype(np.float64)
-                                             for v in (self.norm.y_mean, self.norm.y_std)])).to(self.dev)
+        scale = t.from_numpy(np.concatenate([nm.y_mean, nm.y_std]).astype(np.float64)).to(self.dev)
         f64 = dict(dtype=t.float64, device=self.dev)
         for s in range(0, len(X), chunk):
             Xc = self._x(X[s:s + chunk])
@@ -409,12 +410,36 @@ class Ensemble:
             out[..., s:s + rows, :] = y.cpu().numpy()
         return out
 
+    def _predict_members_numpy(self, X: np.ndarray, chunk: int) -> np.ndarray:
+        """The same for statistics that numpy does not combine in float64, vector by vector (a normaliser
+        fitted to float32 data): in numpy, in its precision."""
+        t = self.torch
+        out = np.empty((len(self.members), len(X), N_OUT))
+        for s in range(0, len(X), chunk):
+            Xc = self._x(X[s:s + chunk])
+            rows = len(Xc)
+            Z = t.empty(rows, N_OUT_PAD, dtype=t.float32, device=self.dev)
+            for i, m in enumerate(self.members):
+                _ensure_rows(m, rows)
+                m.forward(Xc, rows, t.cuda.current_stream().cuda_stream, Z_out=Z)
+                out[i, s:s + rows] = Z[:, :N_OUT].cpu().numpy() * self.norm.y_std + self.norm.y_mean
+        return out
+
     def predict_members(self, X: np.ndarray, chunk: int = 65536) -> np.ndarray:
         """(members, n, 66) raw (de-normalised) outputs."""
         return self._predict(X, chunk, False)
 
     def predict(self, X: np.ndarray) -> np.ndarray:
         return self._predict(X, 65536, True)
+
+
+def _float64_vectors(n: int, data, first, second) -> bool:
+    """Whether numpy combines `data` in float64 with the statistics `first`, then `second`, an element of n at a
+    time: what the device kernels compute. Anything else (float32 or wider types, statistics that broadcast)
+    stays with numpy."""
+    d, a, b = (np.asarray(v).dtype for v in (data, first, second))
+    return (np.shape(first) == (n,) and np.shape(second) == (n,)
+            and np.result_type(d, a) == np.float64 and np.result_type(d, a, b) == np.float64)
 
 
 def _ensure_rows(m: Member, rows: int) -> None:
