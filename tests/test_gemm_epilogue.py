@@ -60,3 +60,33 @@ def test_every_output_of_a_layer(M, N, K, offset):
     assert torch.equal(dXT, dX.t())
     for buf in (xb, db):
         assert _untouched(buf, offset, M * N)
+
+
+@pytest.mark.parametrize("N,K,offset", [(72, 64, 0), (128, 512, 0), (200, 192, 0), (136, 64, 1), (37, 128, 0)])
+def test_few_rows_equal_the_same_rows_of_many(N, K, offset):
+    """A product of few tiles takes narrower ones: the same bits, and both sides of the rule write no more
+    than their matrix. Many rows leave a ragged last tile in either width."""
+    from tissuemc_b200 import surrogate as S
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    across = (N + 127) // 128
+    last_narrow = sms // 2 // across * 128  # the most rows that still take narrow tiles
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    X = torch.randn(last_narrow + 133, K, device="cuda", generator=g).bfloat16()
+    W = (torch.randn(N, K, device="cuda", generator=g) / math.sqrt(K)).bfloat16()
+    bias = torch.randn(N, device="cuda", generator=g)
+    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    got = {}
+    for M in (1, 129, last_narrow, last_narrow + 1, last_narrow + 133):
+        bufs = [_out(M, N, torch.float32, offset), _out(M, N, torch.bfloat16, offset), _out(N, M, torch.bfloat16, offset),
+                _out(M, N, torch.bfloat16, offset), _out(N, M, torch.bfloat16, offset)]
+        (_, Z), (_, H), (_, HT), (_, dX), (_, dXT) = bufs
+        S._call("tmc_b200_nn_linear", S._p(X), S._p(W), S._p(bias), S._p(Z), S._p(H), S._p(HT), M, N, K, 1, s)
+        S._call("tmc_b200_nn_backward_data", S._p(X), S._p(W), S._p(Z), S._p(dX), S._p(dXT), M, N, K, s)
+        for buf, _ in bufs:
+            assert _untouched(buf, offset, M * N)
+        got[M] = Z, H, HT.t(), dX, dXT.t()
+    most = got[last_narrow + 133]
+    for M, outs in got.items():
+        for few, many in zip(outs, most):
+            assert torch.equal(few, many[:M])

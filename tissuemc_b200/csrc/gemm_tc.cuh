@@ -1,6 +1,6 @@
 // D = A * B^T on the 5th-generation tensor cores (tcgen05), BF16 operands, FP32 accumulation in
 // tensor memory, with a fused epilogue. A is M x K and B is N x K, both row-major with K
-// contiguous (K-major), 16-byte aligned; K is a multiple of 64. One CTA of four warps computes a
+// contiguous (K-major), 16-byte aligned; K is a multiple of 64. One CTA of eight warps computes a
 // 128 x BN tile over the K range of its blockIdx.z (split-K: each z covers K / gridDim.z, a
 // multiple of 64):
 //
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_tc_kernel(const __grid_c
         // the ring is free: its last bytes were read by the MMAs that acc_bar waited for
         unsigned char *stage = g.base + warp * kGemmWarpStage;
         static_assert((kGemmThreads / 32) * kGemmWarpStage <= kGemmStages * GemmSmem<BN>::stage_bytes, "staging");
-        static_assert(BN == 128 && kGemmThreads == 256, "eight warps: four row groups x two column halves");
+        static_assert(BN % 64 == 0 && kGemmThreads == 256, "eight warps: four row groups x two column halves");
         const uint32_t lane_addr = g.tmem_d + (static_cast<uint32_t>((warp & 3) * 32) << 16);
 #pragma unroll 1
         for (int c = c_first; c < c_first + BN / 2; c += 32) {

@@ -17,6 +17,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <utility>
 
 #include "../../include/tissuemc_b200.h"
@@ -26,10 +27,10 @@
 namespace tmc {
 namespace {
 
-constexpr int kBN = 128;
+// Columns of a product's tiles (launch_gemm chooses) and of the weight gradients' (the wide ones).
+constexpr int kWide = 128, kNarrow = 64;
 // three stages of 32 KB plus slack: two CTAs per SM, i.e. 2 x 128 of the 512 TMEM columns
-constexpr int kGemmSmemRequest = GemmSmem<kBN>::bytes;
-static_assert(2 * kGemmSmemRequest <= 227 * 1024, "two GEMM CTAs per SM");
+static_assert(2 * GemmSmem<kWide>::bytes <= 227 * 1024, "two GEMM CTAs per SM");
 
 __device__ __forceinline__ float gelu(float x) { return gelu_tanh(x); }
 __device__ __forceinline__ float gelu_grad(float x) { return gelu_tanh_grad(x); }
@@ -616,7 +617,7 @@ __global__ void gate_kernel(const float *__restrict__ Z, int members, size_t mem
 
 std::mutex g_mu;
 int *g_status[64] = {};
-bool g_attr[64] = {};
+int g_gemm_sms[64] = {};  // SMs of a device whose GEMM kernels are ready to launch
 bool g_infer_attr[64] = {};
 int g_infer_clusters[64][kInferMaxMembers + 1] = {};  // clusters of that many CTAs resident at once (-1: none)
 
@@ -663,7 +664,8 @@ int *status_word(int dev) {
 }
 
 template <class Epi> void set_smem_attr() {
-    cudaFuncSetAttribute(gemm_tc_kernel<kBN, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemRequest);
+    cudaFuncSetAttribute(gemm_tc_kernel<kWide, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<kWide>::bytes);
+    cudaFuncSetAttribute(gemm_tc_kernel<kNarrow, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<kNarrow>::bytes);
 }
 
 // cuTensorMapEncodeTiled, from the driver through the runtime (no link against libcuda).
@@ -701,9 +703,9 @@ void launch_chained(void (*kernel)(Params...), dim3 grid, int threads, int smem,
     cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-// What a GEMM launch needs on the current device, under g_mu: the status word, the driver's tensor-map
-// encoder, the kernels' shared memory.
-int gemm_ready(int **status, tmc_status *st) {
+// What a GEMM launch needs on the current device, under g_mu: the status word, the number of SMs, the
+// driver's tensor-map encoder, the kernels' shared memory.
+int gemm_ready(int **status, int *sms, tmc_status *st) {
     const int dev = current_device();
     *status = status_word(dev);
     if (!*status) {
@@ -722,14 +724,27 @@ int gemm_ready(int **status, tmc_status *st) {
         }
         g_encode_tiled = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
     }
-    if (!g_attr[dev]) {
+    if (!g_gemm_sms[dev]) {
         set_smem_attr<EpiF32>();
         set_smem_attr<EpiFwd>();
         set_smem_attr<EpiBwd>();
-        cudaFuncSetAttribute(wgrad_kernel<kBN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemRequest);
-        g_attr[dev] = true;
+        cudaFuncSetAttribute(wgrad_kernel<kWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<kWide>::bytes);
+        cudaDeviceGetAttribute(&g_gemm_sms[dev], cudaDevAttrMultiProcessorCount, dev);
     }
+    *sms = g_gemm_sms[dev];
     return TMC_OK;
+}
+
+// Whether a product's tiles are 64 columns wide instead of 128: while all tiles are on the device at once a
+// product lasts as long as one tile's loads, MMAs and epilogue, and half a tile's are shorter; A is loaded
+// twice as often, though. Up to half as many wide tiles as SMs, so that each narrow one has an SM to itself:
+// last layer at batch 4096 (32 wide tiles) 6.4 -> 5.0 us, a network's gradients at batch 2304 112 -> 93 us, the
+// ensemble's step at batch 1024 0.235 -> 0.209 ms, 2048 0.302 -> 0.290. With the hidden layers at batch 4096
+// (128 tiles) narrow too, one network's gradients go from 147 to 134 us, but the ensemble's step, whose four
+// members fill the device, from 0.412 to 0.434 ms.
+bool narrow_tiles(int M, int N, int splits, int sms) {
+    const int64_t across = (static_cast<int64_t>(N) + kWide - 1) / kWide, down = (static_cast<int64_t>(M) + kGemmBM - 1) / kGemmBM;
+    return 2 * across * down * splits <= sms;
 }
 
 // Common checks and the launch of one tensor-core GEMM (asynchronous).
@@ -753,16 +768,22 @@ int launch_gemm(const void *A, const void *B, int M, int N, int K, const Epi &ep
         return TMC_BAD_ARGUMENT;
     }
     std::lock_guard<std::mutex> lock(g_mu);
-    int *status = nullptr;
-    if (const int rc = gemm_ready(&status, st); rc != TMC_OK) return rc;
+    int *status = nullptr, sms = 0;
+    if (const int rc = gemm_ready(&status, &sms, st); rc != TMC_OK) return rc;
+    const bool narrow = narrow_tiles(M, N, splits, sms);
     CUtensorMap ta, tb;
-    if (!encode_operand(&ta, A, M, K, kGemmBM) || !encode_operand(&tb, B, N, K, kBN)) {
+    if (!encode_operand(&ta, A, M, K, kGemmBM) || !encode_operand(&tb, B, N, K, narrow ? kNarrow : kWide)) {
         put(st, TMC_BAD_ARGUMENT, "tensor-core GEMM operands do not fit a TMA tensor map");
         return TMC_BAD_ARGUMENT;
     }
-    const dim3 grid((N + kBN - 1) / kBN, (M + kGemmBM - 1) / kGemmBM, splits);
-    launch_chained(gemm_tc_kernel<kBN, Epi>, grid, kGemmThreads, kGemmSmemRequest, static_cast<cudaStream_t>(stream), 0, ta,
-                   tb, M, N, K, epi, status, wait_limit, withhold);
+    const auto run = [&](auto bn) {
+        constexpr int BN = decltype(bn)::value;
+        const dim3 grid((N + BN - 1) / BN, (M + kGemmBM - 1) / kGemmBM, splits);
+        launch_chained(gemm_tc_kernel<BN, Epi>, grid, kGemmThreads, GemmSmem<BN>::bytes, static_cast<cudaStream_t>(stream), 0,
+                       ta, tb, M, N, K, epi, status, wait_limit, withhold);
+    };
+    if (narrow) run(std::integral_constant<int, kNarrow>{});
+    else run(std::integral_constant<int, kWide>{});
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         put(st, TMC_CUDA_ERROR, std::string("CUDA error launching the tensor-core GEMM: ") + cudaGetErrorString(e));
@@ -942,23 +963,23 @@ int tmc_b200_nn_weight_grads(const uint16_t *const *A, const uint16_t *const *B,
         return TMC_BAD_CONFIG;
     }
     std::lock_guard<std::mutex> lock(g_mu);
-    int *status = nullptr;
-    if (const int rc = gemm_ready(&status, st); rc != TMC_OK) return rc;
+    int *status = nullptr, sms = 0;
+    if (const int rc = gemm_ready(&status, &sms, st); rc != TMC_OK) return rc;
     WgradProblems P{};
     P.count = count;
     for (int q = 0; q < count; ++q) {
         if (!A[q] || !B[q] || !D[q] || M[q] < 1 || N[q] < 1 || reinterpret_cast<uintptr_t>(A[q]) % 16 != 0 ||
             reinterpret_cast<uintptr_t>(B[q]) % 16 != 0 || !encode_operand(&P.a[q], A[q], M[q], K, kGemmBM) ||
-            !encode_operand(&P.b[q], B[q], N[q], K, kBN)) {
+            !encode_operand(&P.b[q], B[q], N[q], K, kWide)) {
             put(st, TMC_BAD_ARGUMENT, "weight-gradient operands must be 16-byte aligned and fit a TMA tensor map");
             return TMC_BAD_ARGUMENT;
         }
         P.D[q] = D[q];
         P.M[q] = M[q];
         P.N[q] = N[q];
-        P.first[q + 1] = P.first[q] + (M[q] + kGemmBM - 1) / kGemmBM * ((N[q] + kBN - 1) / kBN);
+        P.first[q + 1] = P.first[q] + (M[q] + kGemmBM - 1) / kGemmBM * ((N[q] + kWide - 1) / kWide);
     }
-    launch_chained(wgrad_kernel<kBN>, dim3(static_cast<unsigned>(P.first[count] * splits)), kGemmThreads, kGemmSmemRequest,
+    launch_chained(wgrad_kernel<kWide>, dim3(static_cast<unsigned>(P.first[count] * splits)), kGemmThreads, GemmSmem<kWide>::bytes,
                    static_cast<cudaStream_t>(stream), splits, P, K, splits, status);
     return launched(st);
 }
