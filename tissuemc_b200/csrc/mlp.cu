@@ -397,7 +397,10 @@ __global__ void mse_kernel(const float *__restrict__ pred, const float *__restri
 
 // The loss of a training step with what its backward pass reads: blocks 0 .. row_blocks - 1 take 32 rows
 // of the error each (dZ, its transpose, the loss), the others 32 rows of the network's inputs (their
-// transpose). Three passes and launches in one: 8.0 -> 6.8 us at batch 4096.
+// transpose). Three passes and launches in one: 8.0 -> 6.8 us at batch 4096. A cluster of eight blocks adds its
+// part of the loss at once, in order: float32 atomics round at every sum, in whatever order they come, and
+// with one per 32 rows an epoch's mean loss moved by up to two units in its last place from run to run.
+constexpr uint32_t kMseCluster = 8;
 __global__ void __launch_bounds__(256) mse_transposes_kernel(const float *__restrict__ pred, const float *__restrict__ target,
                                                              __nv_bfloat16 *__restrict__ dZ, __nv_bfloat16 *__restrict__ dZT,
                                                              float *loss, int M, int T, int ld, float scale,
@@ -405,9 +408,10 @@ __global__ void __launch_bounds__(256) mse_transposes_kernel(const float *__rest
                                                              int k, int row_blocks) {
     extern __shared__ __nv_bfloat16 tile[];  // 32 rows of ld or k columns, one apart from a bank multiple
     __shared__ float warp_sum[8];
+    __shared__ float4 part;  // x: the block's part of the loss
     const bool inputs = static_cast<int>(blockIdx.x) >= row_blocks;
     wait_for_inputs();
-    const int row0 = (static_cast<int>(blockIdx.x) - (inputs ? row_blocks : 0)) * 32, rows = min(32, M - row0);
+    const int row0 = (static_cast<int>(blockIdx.x) - (inputs ? row_blocks : 0)) * 32, rows = max(0, min(32, M - row0));
     const int cols = inputs ? k : ld, pitch = cols + 2;
     float l = 0.0f;
     for (int i = threadIdx.x; i < rows * cols; i += 256) {
@@ -434,7 +438,7 @@ __global__ void __launch_bounds__(256) mse_transposes_kernel(const float *__rest
     const int lane = threadIdx.x & 31;
     if (lane < rows)
         for (int c = threadIdx.x >> 5; c < cols; c += 8) out[static_cast<size_t>(c) * M + row0 + lane] = tile[lane * pitch + c];
-    if (inputs) return;  // block-uniform
+    if (inputs) return;  // uniform in a cluster: row_blocks is a multiple of kMseCluster
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
     if (lane == 0) warp_sum[threadIdx.x >> 5] = l;
@@ -442,8 +446,17 @@ __global__ void __launch_bounds__(256) mse_transposes_kernel(const float *__rest
     if (threadIdx.x == 0) {
         float sum = 0.0f;
         for (int w = 0; w < 8; ++w) sum += warp_sum[w];
+        part.x = sum;
+    }
+    __syncwarp();
+    cluster_barrier();  // every block's part is in place
+    if (threadIdx.x == 0 && cluster_rank() == 0) {
+        float sum = 0.0f;
+        for (uint32_t b = 0; b < kMseCluster; ++b) sum += ld_cluster_f32x4(&part, b).x;
         if (sum != 0.0f) atomicAdd(loss, sum * scale);
     }
+    __syncwarp();
+    cluster_barrier();  // no block leaves while its part may still be read
 }
 
 // Polyak averaging of one value: avg = beta avg + (1 - beta) w, with its rounding pinned so that
@@ -1060,9 +1073,9 @@ int tmc_b200_nn_mse_transposes(const float *pred, const float *target, uint16_t 
         put(st, TMC_BAD_ARGUMENT, "NULL argument or bad shape (at most 512 columns)");
         return TMC_BAD_ARGUMENT;
     }
-    const int blocks = (M + 31) / 32;
+    const int clusters = ((M + 31) / 32 + kMseCluster - 1) / kMseCluster, blocks = clusters * kMseCluster;
     launch_chained(mse_transposes_kernel, dim3(static_cast<unsigned>(2 * blocks)), 256,
-                   static_cast<int>(32 * (std::max(ld, k) + 2) * sizeof(__nv_bfloat16)), static_cast<cudaStream_t>(stream), 0,
+                   static_cast<int>(32 * (std::max(ld, k) + 2) * sizeof(__nv_bfloat16)), static_cast<cudaStream_t>(stream), kMseCluster,
                    pred, target, reinterpret_cast<__nv_bfloat16 *>(dZ), reinterpret_cast<__nv_bfloat16 *>(dZT), loss, M, T, ld,
                    scale, reinterpret_cast<const __nv_bfloat16 *>(X), reinterpret_cast<__nv_bfloat16 *>(XT), k, blocks);
     return launched(st);
