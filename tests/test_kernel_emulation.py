@@ -1,0 +1,37 @@
+"""Kernels' own sources on the CPU, every thread a fiber (tests/emulation/kernel_emulator.hpp): interleavings
+that an idle GPU hardly ever shows."""
+
+from __future__ import annotations
+
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+EMULATION = Path(__file__).resolve().parent / "emulation"
+FLAGS = ["-std=c++17", "-O2", "-ffp-contract=off", "-fno-strict-aliasing", "-Wall", "-Wextra", "-Wno-unknown-pragmas"]
+
+
+def _build(source: Path, exe: Path, *flags: str) -> Path:
+    cxx = shutil.which("g++")
+    if cxx is None:
+        pytest.skip("no C++ compiler")
+    subprocess.run([cxx, *FLAGS, *flags, str(source), "-o", str(exe)], check=True)
+    return exe
+
+
+def _run(exe: Path, *args: str) -> None:
+    out = subprocess.run([str(exe), *args], capture_output=True, text=True, timeout=600)
+    assert out.returncode == 0, out.stderr[-2000:]
+
+
+@pytest.fixture(scope="module")
+def small_walks(tmp_path_factory):
+    return _build(EMULATION / "small_walks.cpp", tmp_path_factory.mktemp("emulation") / "small_walks", "-DTMC_FAST_MASK=0")
+
+
+def test_no_photon_is_lost_when_blocks_start_late(small_walks):
+    """1 to 32 lanes a warp, blocks of 1 to 4 warps, some of them starting when others have long claimed
+    their second photons."""
+    _run(small_walks, "late_blocks")

@@ -148,7 +148,7 @@ bool walk_ends_alone(const WalkParams &P, const Plan &pl, bool fast) {
     return fast ? P.photons <= 16 * lanes : P.photons <= lanes / 2;
 }
 
-// How a launch spreads its photons: P.lanes and P.chunk, and the grid (returned). Never more blocks than
+// How a launch spreads its photons: P.lanes, and the grid (returned). Never more blocks than
 // can be resident at once with this plan's shared memory: the kernel is persistent, a second wave would
 // idle. A run whose photons do not fill those is as long as its longest photon, step after step, so the
 // photons go evenly to every SM, to kSmallWarps warps on each before any SM gets more, and a warp's
@@ -165,9 +165,6 @@ int walk_grid(WalkParams &P, const Plan &pl, const void *kern, const cudaDeviceP
     const uint64_t per_sm = std::max((kSmallWarps + warps - 1) / warps, (P.photons + sms * pl.threads - 1) / (sms * pl.threads));
     const uint64_t blocks = std::min({most, sms * per_sm, (P.photons + warps - 1) / warps});
     P.lanes = static_cast<int>(std::min<uint64_t>(32, (P.photons + blocks * warps - 1) / (blocks * warps)));
-    // ids a warp claims at once: one per lane, so that when the ids run out no warp is left holding
-    // a backlog of unstarted photons while others idle
-    P.chunk = P.lanes;
     return static_cast<int>(blocks);
 }
 
@@ -352,7 +349,7 @@ WalkParams make_params(const tmc_run_spec &spec, const tmc_options &opt, const P
     P.profiles = opt.profiles ? 1 : 0;
     P.step_cap = opt.step_cap ? opt.step_cap : kDefaultStepCap;
     P.lanes = 32;  // a small run's launch may use fewer (walk_grid)
-    P.chunk = 32;
+    P.chunk = 32;  // one id per lane: when the ids run out, warps hold few unstarted photons while others idle
     uint32_t k0 = static_cast<uint32_t>(opt.seed), k1 = static_cast<uint32_t>(opt.seed >> 32);
     for (int r = 0; r < 10; ++r) {  // Philox4x32 key schedule (Weyl increments)
         P.round_keys[2 * r] = k0;

@@ -68,8 +68,8 @@ struct WalkParams {
     int batch_smem;        // 1: per-batch totals in shared memory
     int profiles;          // 0: skip A(r,z), R_d(r,a), T_t(r,a)
     uint32_t step_cap;     // a packet still alive after this many steps is ended as an anomaly
-    int lanes;             // lanes of a warp that walk photons (32 unless the run is small: WalkGrid)
-    int chunk;             // photon ids claimed per warp refill (>= lanes)
+    int lanes;             // lanes of a warp that walk photons (32 unless the run is small: walk_grid)
+    int chunk;             // photon ids a warp of 32 lanes claims at once (>= 32); one of fewer: what it needs
     uint32_t round_keys[20];  // Philox key schedule of `seed` (k0, k1 of rounds 0..9), so that the
                               // rounds read their keys from the parameter bank instead of adding
     LayerC layers[kMaxLayers];

@@ -166,7 +166,6 @@ template <int FAST, bool CORE, bool PROF> __device__ __noinline__ void walk_park
     PlainCtx<FAST, CORE, PROF> C = plain_ctx<FAST, CORE, PROF>(P, S, smem);
     AloneState &A = *reinterpret_cast<AloneState *>(smem + S.alone);
     const unsigned lane = threadIdx.x & 31u;
-    const int warps = static_cast<int>(P.threads) / 32;
     AloneTables &T = alone_tables(smem + S.ring, threadIdx.x >> 5);
     for (;;) {
         Lane M;
@@ -216,6 +215,7 @@ __device__ __forceinline__ void walk_body(const WalkParams &P) {
     bool held = false;  // L holds a photon whose totals are not yet published
     Lane L;
     const int alone_at = alone_per_warp<FAST>() * static_cast<int>(P.threads / 32u);
+    static_assert(kAlonePerWarp * 8 < 32, "a block with a full warp does not turn to walking alone");
 
     for (;;) {
         // ---- relaunch: lanes without a photon take the next ids from the warp's pool
@@ -228,12 +228,15 @@ __device__ __forceinline__ void walk_body(const WalkParams &P) {
             const uint32_t n = static_cast<uint32_t>(__popc(need));
             const uint32_t rank = static_cast<uint32_t>(__popc(need & lt_mask));
             uint32_t base = 0u;
-            if (pool.must_claim(n)) {  // one lane claims the next chunk for the warp
+            // a run too small to fill its warps' lanes claims no more ids than it launches now: what a warp
+            // held in its pool, the idle lanes of others could have walked
+            const uint32_t claim = P.lanes < 32 ? n : chunk;
+            if (pool.must_claim(n)) {  // one lane claims the next ids for the warp
                 const int leader = __ffs(need) - 1;
-                if (static_cast<int>(lane) == leader) base = atomicAdd(P.counter, chunk);
+                if (static_cast<int>(lane) == leader) base = atomicAdd(P.counter, claim);
                 base = __shfl_sync(0xffffffffu, base, leader);
             }
-            const uint32_t my = pool.take(n, rank, base, chunk);
+            const uint32_t my = pool.take(n, rank, base, claim);
             const bool mine = (need >> lane) & 1u;
             ex_mask |= __ballot_sync(0xffffffffu, mine && my >= n_photons);
             if (mine && my < n_photons) {
@@ -244,7 +247,10 @@ __device__ __forceinline__ void walk_body(const WalkParams &P) {
             }
         }
         if constexpr (ALONE) {
-            if (ex_mask) {  // ids have run out (or the run is small): few enough packets to walk alone?
+            // Ids have run out (or the run is small): few enough packets to walk alone? A warp that leaves holds
+            // no id that it has not launched: with all 32 lanes walking, a lane is exhausted only after the
+            // pool's last id, and 32 live lanes are too many; with fewer, the pool never holds any.
+            if (ex_mask) {
                 if (lane == 0) A.live[threadIdx.x >> 5] = static_cast<unsigned char>(__popc(~ex_mask));
                 if (live_lanes(A) <= alone_at) break;
             }
