@@ -233,6 +233,9 @@ int main(int argc, char **argv) {
         walks<1>({0, 2}, emu::Order::Lockstep, 4, kNoCap);
         walks<0>({0, 2}, emu::Order::Lockstep, 4, kNoCap);
         walks<1>({0, 2}, emu::Order::Lockstep, 1, 7u);
+    } else if (what == "layer_changes") {
+        walks<1>({1}, emu::Order::Lockstep, 2, kNoCap);
+        walks<0>({1}, emu::Order::Lockstep, 2, kNoCap);
     } else {
         std::fprintf(stderr, "no such case\n");
         return 2;

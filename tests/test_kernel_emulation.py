@@ -35,3 +35,9 @@ def test_no_photon_is_lost_when_blocks_start_late(small_walks):
     """1 to 32 lanes a warp, blocks of 1 to 4 warps, some of them starting when others have long claimed
     their second photons."""
     _run(small_walks, "late_blocks")
+
+
+def test_packets_walked_alone_through_thin_layers(small_walks):
+    """Boundary after boundary, with nothing scored in between: the layer's tables are rewritten only when
+    every lane of the warp has read the last one's."""
+    _run(small_walks, "layer_changes")

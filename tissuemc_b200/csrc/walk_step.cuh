@@ -670,7 +670,10 @@ template <int FAST, class Base> struct AloneCtx {
         return more;
     }
     __device__ __forceinline__ void leave_layer(Lane &L) { score(L); }
-    __device__ __forceinline__ void enter_layer(Lane &L) { steps_of(L); }
+    __device__ __forceinline__ void enter_layer(Lane &L) {
+        __syncwarp();  // every lane has read its free path (score() has no barrier when it has no records)
+        steps_of(L);
+    }
 };
 
 // How many live lanes each warp of a block has, and the next parked packet to take (shared memory).
