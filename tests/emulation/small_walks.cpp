@@ -236,6 +236,18 @@ int main(int argc, char **argv) {
     } else if (what == "layer_changes") {
         walks<1>({1}, emu::Order::Lockstep, 2, kNoCap);
         walks<0>({1}, emu::Order::Lockstep, 2, kNoCap);
+    } else if (what == "lanes_apart") {
+        walks<1>({0, 1, 2}, emu::Order::Skewed, 1, kNoCap);
+        walks<0>({0, 1, 2}, emu::Order::Skewed, 1, kNoCap);
+    } else if (what == "sweep_lanes_apart") {
+        uint64_t seed = 1;
+        for (emu::Order order : {emu::Order::Lockstep, emu::Order::Skewed})
+            for (int threads : {32, 64, 128})
+                for (uint32_t lanes : {1u, 7u, 32u})
+                    for (uint32_t chunk : {1u, 13u, 40u}) {
+                        sweep_case<1>({40, 1, 23, 9}, 3, threads, chunk, lanes, order, ++seed);
+                        sweep_case<0>({5, 60, 2}, 2, threads, chunk, lanes, order, ++seed);
+                    }
     } else {
         std::fprintf(stderr, "no such case\n");
         return 2;

@@ -41,3 +41,10 @@ def test_packets_walked_alone_through_thin_layers(small_walks):
     """Boundary after boundary, with nothing scored in between: the layer's tables are rewritten only when
     every lane of the warp has read the last one's."""
     _run(small_walks, "layer_changes")
+
+
+@pytest.mark.parametrize("case", ["lanes_apart", "sweep_lanes_apart"])
+def test_lanes_of_a_warp_leave_the_step_loop_together(small_walks, case):
+    """Lanes scheduled independently: each reads the block's counts of live lanes at its own time, while other
+    warps write them."""
+    _run(small_walks, case)

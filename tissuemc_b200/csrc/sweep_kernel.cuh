@@ -500,7 +500,7 @@ template <int FAST> __global__ void TMC_SWEEP_BOUNDS sweep_block_kernel(const __
         }
         if (done) {  // no chunk is left: few enough packets to walk alone?
             if (lane == 0) S.alone.live[threadIdx.x >> 5] = static_cast<unsigned char>(__popc(~ex_mask));
-            if (live_lanes(S.alone) <= alone_at) break;
+            if (__any_sync(0xffffffffu, live_lanes(S.alone) <= alone_at)) break;  // one decision for the warp
         }
         top_up<FAST>(L, C, alive);
         if (!alive) continue;

@@ -252,7 +252,9 @@ __device__ __forceinline__ void walk_body(const WalkParams &P) {
             // pool's last id, and 32 live lanes are too many; with fewer, the pool never holds any.
             if (ex_mask) {
                 if (lane == 0) A.live[threadIdx.x >> 5] = static_cast<unsigned char>(__popc(~ex_mask));
-                if (live_lanes(A) <= alone_at) break;
+                // (one decision for the warp: the lanes read the counts while other warps write them. Counts
+                // only fall, so whoever sees few enough first decides for all)
+                if (__any_sync(0xffffffffu, live_lanes(A) <= alone_at)) break;
             }
         } else {
             if (ex_mask == 0xffffffffu) break;  // exhausted lanes hold no photon: the warp is done
