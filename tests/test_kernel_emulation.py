@@ -48,3 +48,12 @@ def test_lanes_of_a_warp_leave_the_step_loop_together(small_walks, case):
     """Lanes scheduled independently: each reads the block's counts of live lanes at its own time, while other
     warps write them."""
     _run(small_walks, case)
+
+
+def test_gemm_roles_give_up_together(tmp_path):
+    """Waits of the tensor-core GEMM that run out while some lanes of the warp see their barrier complete."""
+    shutil.copy(EMULATION.parents[1] / "tissuemc_b200/csrc/gemm_tc.cuh", tmp_path / "gemm_tc.cuh")
+    shutil.copy(EMULATION / "umma_stub.hpp", tmp_path / "umma.cuh")
+    for header in ("cuda.h", "cuda_bf16.h"):
+        (tmp_path / header).write_text("")
+    _run(_build(EMULATION / "gemm_waits.cpp", tmp_path / "gemm_waits", f"-I{tmp_path}"))

@@ -56,6 +56,12 @@ template <int BN> struct GemmCta {
     uint32_t tmem_d;
 };
 
+// A whole warp's bounded wait: true when every lane saw the phase complete. Lanes poll, and give up, at their
+// own times; the warp goes on, or gives up, as one (its next elect.sync names all 32 lanes).
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, uint32_t limit) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit)) != 0;
+}
+
 // Barriers, TMEM and the bias of columns n0 .. (zeros past N or without one). Whole CTA.
 template <int BN>
 __device__ __forceinline__ GemmCta<BN> gemm_begin(unsigned char *raw, const float *bias, int n0, int N) {
@@ -102,7 +108,7 @@ __device__ __forceinline__ void gemm_products(const GemmCta<BN> &g, const CUtens
             const int s = kt % kGemmStages;
             // the stage was last read by the MMAs of slice kt - kGemmStages
             if (kt >= kGemmStages &&
-                !mbar_wait(&g.empty[s], static_cast<uint32_t>((kt / kGemmStages - 1) & 1), wait_limit)) {
+                !warp_wait(&g.empty[s], static_cast<uint32_t>((kt / kGemmStages - 1) & 1), wait_limit)) {
                 ok = false;
                 break;
             }
@@ -117,7 +123,7 @@ __device__ __forceinline__ void gemm_products(const GemmCta<BN> &g, const CUtens
         }
         // every load issued has landed before the CTA can end (the last phase of each stage)
         for (int kt = issued > kGemmStages ? issued - kGemmStages : 0; kt < issued; ++kt)
-            if (!mbar_wait(&g.full[kt % kGemmStages], static_cast<uint32_t>((kt / kGemmStages) & 1), kGemmDrainLimit)) {
+            if (!warp_wait(&g.full[kt % kGemmStages], static_cast<uint32_t>((kt / kGemmStages) & 1), kGemmDrainLimit)) {
                 ok = false;
                 if (lane == 0) atomicExch(status, 2);
             }
@@ -125,7 +131,7 @@ __device__ __forceinline__ void gemm_products(const GemmCta<BN> &g, const CUtens
         // ---- issuer: the whole warp waits, one lane issues the MMAs and the commits
         for (int kt = 0; kt < kt_n; ++kt) {
             const int s = kt % kGemmStages;
-            if (!mbar_wait(&g.full[s], static_cast<uint32_t>((kt / kGemmStages) & 1), wait_limit)) {
+            if (!warp_wait(&g.full[s], static_cast<uint32_t>((kt / kGemmStages) & 1), wait_limit)) {
                 ok = false;
                 break;
             }
@@ -151,10 +157,10 @@ __device__ __forceinline__ void gemm_products(const GemmCta<BN> &g, const CUtens
 // Whole CTA: every MMA issued has completed (before TMEM is read or released); false when a wait gave up.
 template <int BN> __device__ __forceinline__ bool gemm_done(const GemmCta<BN> &g, int *status, uint32_t wait_limit) {
     const int lane = threadIdx.x & 31;
-    if (!mbar_wait(g.acc_bar, 0u, wait_limit)) {
+    if (!warp_wait(g.acc_bar, 0u, wait_limit)) {
         if (lane == 0) atomicCAS(status, 0, 1);
         *g.abort_flag = 1;
-        if (!mbar_wait(g.acc_bar, 0u, kGemmDrainLimit) && lane == 0) atomicExch(status, 2);
+        if (!warp_wait(g.acc_bar, 0u, kGemmDrainLimit) && lane == 0) atomicExch(status, 2);
     }
     tc_fence_after();
     __syncthreads();  // orders the abort flag: the epilogue runs in every warp or none
