@@ -143,9 +143,9 @@ uint64_t resident_blocks(const void *kern, const cudaDeviceProp &prop, int threa
 // 2,844; skin5 1.3 3.06 / 4.46 ms, 6.6 7.25 / 8.20, 13 12.6 / 13.2, 66 55.7 / 54.2. In exact math the
 // accurate functions are most of a step either way: three layers, 0.07 a lane 380 / 501 us, 0.2 480 / 581,
 // 0.66 816 / 773.
-bool walk_ends_alone(const WalkParams &P, const Plan &pl, bool fast) {
+bool walk_ends_alone(uint64_t photons, const Plan &pl, bool fast) {
     const uint64_t lanes = static_cast<uint64_t>(pl.grid) * static_cast<uint64_t>(pl.threads);
-    return fast ? P.photons <= 16 * lanes : P.photons <= lanes / 2;
+    return fast ? photons <= 16 * lanes : photons <= lanes / 2;
 }
 
 // How a launch spreads its photons: P.lanes, and the grid (returned). Never more blocks than
@@ -367,9 +367,10 @@ namespace {
 // (zeroed here; a word no other launch in flight uses). Records ev0/ev1 around it if given.
 // With count > 0, only photons [first, first + count) of the run are walked (a shard: the same
 // streams and batches as in the whole run, so the shards' tallies add up to the run's).
+// With stands_for > 0, the launch is a sample of a run of that many photons and takes that run's kernel.
 void launch_walk(const tmc_run_spec &spec, const tmc_options &opt, DeviceCtx &c,
                  unsigned long long *d_tally, unsigned long long *counter, cudaStream_t stream, cudaEvent_t e0,
-                 cudaEvent_t e1, uint64_t first = 0, uint64_t count = 0) {
+                 cudaEvent_t e1, uint64_t first = 0, uint64_t count = 0, uint64_t stands_for = 0) {
     const RunShape sh = shape_of(spec, opt);
     const size_t words = tally_offsets(sh).total;
     const int threads = opt.threads_per_block > 0 ? opt.threads_per_block : 256;
@@ -384,7 +385,7 @@ void launch_walk(const tmc_run_spec &spec, const tmc_options &opt, DeviceCtx &c,
     if (smem > c.prop.sharedMemPerBlockOptin)
         throw Fail(TMC_BAD_CONFIG, "the tally plan does not fit in shared memory");
     const void *kern = walk_kernel_for(opt.fast_math != 0, pl.tr_a > 0 && pl.tz_a > 0, P.profiles != 0,
-                                       walk_ends_alone(P, pl, opt.fast_math != 0));
+                                       walk_ends_alone(stands_for ? stands_for : P.photons, pl, opt.fast_math != 0));
     const int grid = walk_grid(P, pl, kern, c.prop, smem);
     if (e0) TMC_CUDA(cudaEventRecord(e0, stream));
     if (counter == d_tally + words) {  // one clear for both
@@ -625,7 +626,7 @@ int tmc_b200_run_static(const tmc_run_spec *spec, const tmc_options *opt, tmc_re
         if (smem > d.prop.sharedMemPerBlockOptin)
             throw Fail(TMC_BAD_CONFIG, "the tally plan does not fit in shared memory");
         const void *kern = walk_kernel_for(opt->fast_math != 0, pl.tr_a > 0 && pl.tz_a > 0, P.profiles != 0,
-                                           walk_ends_alone(P, pl, opt->fast_math != 0));
+                                           walk_ends_alone(P.photons, pl, opt->fast_math != 0));
         const int grid = walk_grid(P, pl, kern, d.prop, smem);
         // the array keeps the previous call's contents: the counter and the tallies start at zero
         TMC_CUDA(cudaMemsetAsync(d.scratch, 0, (kStaticHeadWords + words) * 8, 0));
@@ -683,7 +684,9 @@ int tmc_b200_autotune(const tmc_run_spec *spec, tmc_options *opt, uint64_t sampl
                 return 1e30;  // not a plan this device can run
             double best = 1e30;
             for (int rep = 0; rep < 3; ++rep) {  // a warm-up, then the best of two
-                launch_walk(*spec, o, c, c.d_tally, c.d_counter, c.stream, c.ev0, c.ev1);
+                // the kernel that the whole run will take: the one for small runs prefers other plans (the slab
+                // tuned on 1e6 photons with it: 2e7 photons 5.86 ms; with this one 5.53, as by default)
+                launch_walk(*spec, o, c, c.d_tally, c.d_counter, c.stream, c.ev0, c.ev1, 0, 0, total);
                 TMC_CUDA(cudaStreamSynchronize(c.stream));
                 float ms = 0.f;
                 TMC_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
