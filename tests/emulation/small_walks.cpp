@@ -32,6 +32,8 @@ const Tissue kTissues[] = {
     {"thin layers", {{1.4f, 5.0f, 60.0f, 0.8f, 0.004f}, {1.4f, 2.0f, 5.0f, 0.0f, 0.003f}, {1.5f, 9.0f, 40.0f, 0.7f, 0.002f},
                      {1.5f, 1.0f, 3.0f, -0.3f, 0.003f}, {1.3f, 4.0f, 90.0f, 0.9f, 0.01f}}},
     {"thick", {{1.37f, 12.0f, 90.0f, 0.7f, 1.0f}}},
+    // mua = 1e-46 and d = 1e39 in float32 (both are accepted): every score is no number, until the step cap
+    {"clear and endless", {{1.0f, 0.0f, 0.0f, 0.0f, INFINITY}}},
 };
 constexpr int kNz = 6, kNr = 5, kNa = 3;
 constexpr uint32_t kNoCap = 2000000000u;
@@ -236,6 +238,9 @@ int main(int argc, char **argv) {
     } else if (what == "layer_changes") {
         walks<1>({1}, emu::Order::Lockstep, 2, kNoCap);
         walks<0>({1}, emu::Order::Lockstep, 2, kNoCap);
+    } else if (what == "no_numbers") {
+        walks<1>({3}, emu::Order::Lockstep, 2, 23u);
+        walks<0>({3}, emu::Order::Lockstep, 2, 20u);
     } else if (what == "lanes_apart") {
         walks<1>({0, 1, 2}, emu::Order::Skewed, 1, kNoCap);
         walks<0>({0, 1, 2}, emu::Order::Skewed, 1, kNoCap);

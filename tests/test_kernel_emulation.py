@@ -43,6 +43,11 @@ def test_packets_walked_alone_through_thin_layers(small_walks):
     _run(small_walks, "layer_changes")
 
 
+def test_scores_that_are_no_numbers(small_walks):
+    """A packet walked alone sums its scores as a lane does, also where each is no number (2^63)."""
+    _run(small_walks, "no_numbers")
+
+
 @pytest.mark.parametrize("case", ["lanes_apart", "sweep_lanes_apart"])
 def test_lanes_of_a_warp_leave_the_step_loop_together(small_walks, case):
     """Lanes scheduled independently: each reads the block's counts of live lanes at its own time, while other

@@ -598,10 +598,11 @@ template <int FAST, class Base> struct AloneCtx {
             B.absorb(T.xy[lane], T.z[lane], v);
         }
         L.anomalies += static_cast<uint32_t>(__popc(__ballot_sync(0xffffffffu, bad)));
-        // the sum of the values, each at most 10 * 2^32: 24 bits and the rest apart
+        // the sum of the values, 24 bits at a time and what is left of 64 (a weight that is no number is 2^63)
         const uint32_t lo = __reduce_add_sync(0xffffffffu, static_cast<uint32_t>(v) & 0xFFFFFFu);
-        const uint32_t hi = __reduce_add_sync(0xffffffffu, static_cast<uint32_t>(v >> 24));
-        L.run_abs += (static_cast<unsigned long long>(hi) << 24) + lo;
+        const uint32_t mid = __reduce_add_sync(0xffffffffu, static_cast<uint32_t>(v >> 24) & 0xFFFFFFu);
+        const uint32_t hi = __reduce_add_sync(0xffffffffu, static_cast<uint32_t>(v >> 48));
+        L.run_abs += (static_cast<unsigned long long>(hi) << 48) + (static_cast<unsigned long long>(mid) << 24) + lo;
         records = 0;
         __syncwarp();
     }
