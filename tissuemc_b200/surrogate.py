@@ -435,10 +435,11 @@ class Ensemble:
 
 def _float64_vectors(n: int, data, first, second) -> bool:
     """Whether numpy combines `data` in float64 with the statistics `first`, then `second`, an element of n at a
-    time: what the device kernels compute. Anything else (float32 or wider types, statistics that broadcast)
-    stays with numpy."""
-    d, a, b = (np.asarray(v).dtype for v in (data, first, second))
-    return (np.shape(first) == (n,) and np.shape(second) == (n,)
+    time: what the device kernels compute. Anything else (float32 or wider types, statistics that broadcast,
+    array classes with an arithmetic of their own, such as masked arrays) stays with numpy."""
+    v = [np.asanyarray(x) for x in (data, first, second)]
+    d, a, b = (x.dtype for x in v)
+    return (all(type(x) in (np.ndarray, np.memmap) for x in v) and np.shape(first) == (n,) and np.shape(second) == (n,)
             and np.result_type(d, a) == np.float64 and np.result_type(d, a, b) == np.float64)
 
 
