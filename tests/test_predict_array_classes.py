@@ -34,3 +34,10 @@ def test_network_inputs_of_every_array_class_are_numpys(tmp_path):
         Xn = np.zeros((40, S.K_IN), np.float32)
         Xn[:, :13] = (X - mean) / std
         assert torch.equal(ens._x(X), torch.from_numpy(Xn).cuda().bfloat16()), name
+
+
+@pytest.mark.gpu
+def test_predict_members_of_no_members_is_empty():
+    ens = S.Ensemble(members=0, batch=256)
+    ens.norm = S.Norm(np.zeros(13), np.ones(13), np.zeros(66), np.ones(66))
+    assert ens.predict_members(np.zeros((5, 13))).shape == (0, 5, S.N_OUT)

@@ -390,7 +390,7 @@ class Ensemble:
     def _predict(self, X: np.ndarray, chunk: int, mean: bool) -> np.ndarray:
         """Raw (de-normalised) outputs in float64: every member's (members, n, 66), or their mean (n, 66)."""
         t, M, nm = self.torch, len(self.members), self.norm
-        if not _float64_vectors(N_OUT, np.float32(0), nm.y_std, nm.y_mean):
+        if M == 0 or not _float64_vectors(N_OUT, np.float32(0), nm.y_std, nm.y_mean):
             return self._predict_members_numpy(X, chunk).mean(0) if mean else self._predict_members_numpy(X, chunk)
         out = np.empty((len(X), N_OUT) if mean else (M, len(X), N_OUT))
         scale = t.from_numpy(np.concatenate([nm.y_mean, nm.y_std]).astype(np.float64)).to(self.dev)
