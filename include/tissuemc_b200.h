@@ -184,8 +184,10 @@ TMC_B200_API int tmc_b200_run_device_range(const tmc_run_spec *spec, const tmc_o
 TMC_B200_API int tmc_b200_decode(const tmc_run_spec *spec, const tmc_options *opt, const uint64_t *raw,
                     tmc_result *result, tmc_status *status);
 
-/* Launch and shared-memory plan of a walk: block size, blocks per SM, grid, the shared tiles of
- * A(r,z) (core rows tr_a x depth bins tz_a, plus the clamped last row and column when cross = 1),
+/* Launch and shared-memory plan of a walk: block size, blocks per SM, grid (those of a long run: a
+ * launch takes no more blocks than its photons fill, and a run short enough that its last packets are
+ * walked alone no more than that kernel's registers allow), the shared tiles of A(r,z) (core rows
+ * tr_a x depth bins tz_a, plus the clamped last row and column when cross = 1),
  * the shared rows of R_d(r,a) and T_t(r,a), whether the per-batch totals are in shared memory, and
  * the dynamic shared memory per block in bytes. */
 typedef struct {
@@ -205,7 +207,8 @@ TMC_B200_API int tmc_b200_plan(const tmc_run_spec *spec, const tmc_options *opt,
  * T_t(r,a), the shared "cross" of A(r,z)) by coordinate descent on a sample of the run
  * (min(photons, sample_photons) photons, the run's seed and batches), each the best of two timed
  * launches after one warm-up, and write the fastest into opt's threads_per_block, blocks_per_sm,
- * tile_tz, tile_ra_rows and tile_cross. The results of a run do not depend on the plan (integer
+ * tile_tz, tile_ra_rows and tile_cross. The sample runs the kernel that the whole run will take; one too
+ * small to fill the device still weighs the run's end more than the run does. The results of a run do not depend on the plan (integer
  * tallies). plan (optional) receives the chosen plan; default_seconds and best_seconds (optional)
  * the sample's kernel time with the planner's default plan and with the chosen one. Replaces the
  * fixed occupancy sizing of the reference's GPU engine (src/cuda/engine.cu:216-239). */
@@ -263,7 +266,9 @@ typedef struct {
     int32_t profiles;          /* 0: totals only */
     int32_t device;
     int32_t threads_per_block; /* 0 = 256 */
-    int32_t item_photons;      /* photons per work-queue item; 0 = 256 */
+    int32_t item_photons;      /* 0 = 256. Totals only, or with a tile: photons per work-queue item. Otherwise
+                                  blocks take chunks of a configuration's photons, sized by the estimate of
+                                  its cost (at least 32) but never above 8 * item_photons */
     int32_t tile_r, tile_z;    /* per-warp shared-memory tile of A(r,z): the first tile_r x tile_z
                                   bins of the configuration of the warp's current item (0 x 0 =
                                   none, the default; at most 32 KB of tiles per block) */
@@ -277,7 +282,7 @@ typedef struct {
 } tmc_sweep_sizes;
 
 /* Options for the sweep workload of this engine's benchmark: grid nr = nz = 64, dr = dz = 0.01 cm,
- * na = 1, 10 batches, fast math, 256 threads, 256 photons per item. */
+ * na = 1, 10 batches, fast math, 256 threads, item_photons 256. */
 TMC_B200_API void tmc_b200_sweep_default_options(tmc_sweep_options *opt);
 
 /* Draw n configurations: 1-3 layers sharing one refractive index n ~ U[1.33, 1.5] in air;

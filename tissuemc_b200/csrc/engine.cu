@@ -85,7 +85,9 @@ cudaError_t allow_walk_smem(const cudaDeviceProp &prop) {
 }
 
 // Blocks per SM the registers of the walk kernel allow: the instantiation without a core tile when
-// the options rule the core tile out (tile_tz = -1), else the one with it (the larger of the two).
+// the options rule the core tile out (tile_tz = -1), else the one with it (the larger of the two). It is the
+// kernel of long runs whatever the run's size: a run whose last packets are walked alone has the same plan and
+// launches the blocks that its own kernel fits (walk_grid).
 int walk_blocks_per_sm(bool fast, int threads, bool core) {
     int bps = 0;
     const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, walk_kernel_for(fast, core), threads, 0);

@@ -698,8 +698,8 @@ bool encode_operand(CUtensorMap *map, const void *ptr, int rows, int K, int box_
 
 // A launch that may start under the kernel before it in its stream (umma.cuh, wait_for_inputs): the kernels
 // of a training step are a few microseconds long, a good part of it their start. With it one
-// network's gradients at batch 4096 165 -> 146 us, an ensemble step at batch 1024 0.244 -> 0.234 ms, at 4096
-// 0.415 -> 0.412 ms.
+// network's gradients at batch 4096 165 -> 146 us, an ensemble step (in epochs of 16 steps) at batch 1024
+// 0.244 -> 0.234 ms, at 4096 0.415 -> 0.412 ms.
 template <class... Params, class... Args>
 void launch_chained(void (*kernel)(Params...), dim3 grid, int threads, int smem, cudaStream_t s, int cluster, Args &&...args) {
     cudaLaunchConfig_t cfg{};
@@ -754,7 +754,7 @@ int gemm_ready(int **status, int *sms, tmc_status *st) {
 // last layer at batch 4096 (32 wide tiles) 6.4 -> 5.0 us, a network's gradients at batch 2304 112 -> 93 us, the
 // ensemble's step at batch 1024 0.235 -> 0.209 ms, 2048 0.302 -> 0.290. With the hidden layers at batch 4096
 // (128 tiles) narrow too, one network's gradients go from 147 to 134 us, but the ensemble's step, whose four
-// members fill the device, from 0.412 to 0.434 ms.
+// members fill the device, from 0.412 to 0.434 ms (in epochs of 16 steps).
 bool narrow_tiles(int M, int N, int splits, int sms) {
     const int64_t across = (static_cast<int64_t>(N) + kWide - 1) / kWide, down = (static_cast<int64_t>(M) + kGemmBM - 1) / kGemmBM;
     return 2 * across * down * splits <= sms;

@@ -9,7 +9,7 @@
 // options ask for a tile of A(r,z) per warp; what follows here is the kernel for that and for totals only.
 //
 // Work is a queue of items (configuration, first photon, count): configuration c's photons in
-// chunks of item_photons, numbered through a prefix sum and taken band by band, in a strided
+// items of item_photons, numbered through a prefix sum and taken band by band, in a strided
 // permutation inside each band (work_queue.cuh, SweepOrder), so that the warps at work at any
 // moment are spread over many configurations (their tallies then rarely meet on one L2 line). The
 // host lays the configurations out longest photons first, so the bands run from the configurations
@@ -52,9 +52,9 @@ static_assert(sizeof(SweepConfigC) == 128, "SweepConfigC layout");
 struct SweepHeader {
     uint32_t blocks, lanes; // block kernel: blocks at work, and lanes of each warp (fewer in a small sweep)
     uint32_t n_cfg;         // configurations
-    uint32_t item_photons;  // photons per item (the last item of a configuration may hold fewer)
-    SweepOrder order;       // order.total items (configuration c has ceil(photons_c / item_photons))
-                            // and the order in which they are taken
+    uint32_t item_photons;  // item kernel: photons per item (the last item of a configuration may hold fewer)
+    SweepOrder order;       // order.total items (configuration c has ceil(photons_c / item_photons); block
+                            // kernel: its chunks) and the order in which they are taken
 };
 
 struct SweepParams {
@@ -74,9 +74,10 @@ struct SweepParams {
     int tile_words;                 // block kernel: the block's shared tile, the first words of A(r,z)
 };
 
-// 1: an ended packet's totals are published when its lane relaunches (as in the single-run kernel)
-// instead of in the step; measured 0.9 % slower with one step per pass and 0.5 % faster with three
-// (within the noise, and the kernel spills), so 0
+// The item kernel (a tile per warp, or totals only). 1: an ended packet's totals are published when its lane
+// relaunches (as in the other kernels) instead of in the step. Measured on 1,024 sampled configurations: totals only
+// 239.3 ms with 0, 237.4 with 1, tiles of 8 x 8 511 and 510; left at 0, as it came out ahead or level in
+// earlier forms of the loop
 #ifndef TMC_SWEEP_PUBLISH_AT_RELAUNCH
 #define TMC_SWEEP_PUBLISH_AT_RELAUNCH 0
 #endif

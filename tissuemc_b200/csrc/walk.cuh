@@ -6,12 +6,13 @@
 // (include/tissuemc/philox.hpp:49-57, 91-122, 133-136), so photon i sees the same random words as
 // on the CPU. The structure is this engine's own:
 //
-//  * a lane is one thread of a persistent, warp-synchronous loop; a lane whose photon ends claims
-//    the next id from a per-warp pool, which the warp refills from a global counter in chunks;
+//  * a lane is one thread of a persistent, warp-synchronous loop; a lane whose photon ends takes
+//    the next id from a per-warp pool, which the warp refills from a global counter 32 ids at a time
+//    (in a run too small to use every lane, a warp claims just the ids it needs);
 //  * all photon state and the hot constants of the current layer live in registers; the random
-//    words wait in a 16-word ring per lane in shared memory (walk_step.cuh, Ring), refilled with
-//    one Philox block by every lane of the warp with room for it whenever any lane has fewer than
-//    the four a step may draw; the layer table lives in shared memory and is read only when a
+//    words wait in a 16-word ring per lane in shared memory (walk_step.cuh, Ring), topped up before
+//    every pass of the loop, Philox block by block by every lane of the warp with room for one, while
+//    any lane has fewer than the pass's steps may draw (top_up); the layer table lives in shared memory and is read only when a
 //    packet changes layer or meets a boundary;
 //  * every tally is an unsigned 64-bit fixed-point integer (weight * 2^32, rounded), so sums are
 //    exact and a run's output does not depend on scheduling; per-photon values (events, absorbed
