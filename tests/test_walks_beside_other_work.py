@@ -12,8 +12,8 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-# one photon short of, and at, a lane more per warp of 148 blocks; fast math walks alone from 16 packets a
-# block, exact math from 8
+# 3 to 16 lanes a warp in 148 blocks of 8 warps in fast math, 2 to 8 in exact math: more than a block walks alone
+# from the start, but few enough for one warp's lanes alone to be below the limit (16 packets a block, 8)
 @pytest.mark.parametrize("fast, photons", [(True, 2500), (True, 3552), (True, 5000), (True, 10_000), (True, 18_944),
                                            (False, 1500), (False, 2369), (False, 9000)])
 def test_small_walk_beside_a_large_one(fast, photons):
